@@ -315,19 +315,6 @@ __global__ void small_fft_kernel(SmallCols t, uint32_t n, int inverse) {
   for (uint32_t k = 0; k < (1u << ld); k++) t.dst[i][k] = v[k];
 }
 
-// In-place bit reversal: thread i swaps i <-> rev(i) when i < rev(i).
-__global__ void bit_reverse_kernel(uint32_t* v, uint32_t log_n) {
-  uint64_t n = 1ull << log_n;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t j = __brevll(i) >> (64 - log_n);
-    if (i < j) {
-      uint32_t a = v[i], b = v[j];
-      v[i] = b;
-      v[j] = a;
-    }
-  }
-}
-
 // Integer-issue ceiling of the butterfly (no reference counterpart): every
 // thread applies `iters` rounds of 5 layers x 16 forward butterflies (bfly2,
 // the pass kernels' arithmetic) to 32 values held in registers, with one
@@ -355,12 +342,12 @@ __global__ void __launch_bounds__(256) butterfly_probe_kernel(uint32_t iters, ui
   if (x == 0x12345678u) out[0] = x;  // keeps the chain live
 }
 
-// Bit reversal of up to kFftMaxCols columns of one size in one launch
-// (blockIdx.y = column): out of place (dst[brev(i)] = src[i], coalesced
-// reads), or in place by pairwise swaps when dst == src.
+// Bit reversal of up to kFftMaxCols columns of one size below 2^10 in one
+// launch (blockIdx.y = column): out of place (dst[brev(i)] = src[i]), or in
+// place by pairwise swaps when dst == src.
 __global__ void bit_reverse_cols_kernel(FftCols t, uint32_t log_n) {
   const uint64_t n = 1ull << log_n;
-  const uint32_t* __restrict__ src = t.src[blockIdx.y];
+  const uint32_t* src = t.src[blockIdx.y];
   uint32_t* dst = t.dst[blockIdx.y];
   const bool in_place = src == dst;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -372,6 +359,41 @@ __global__ void bit_reverse_cols_kernel(FftCols t, uint32_t log_n) {
       dst[i] = b;
       dst[j] = a;
     }
+  }
+}
+
+// The same for columns of at least 2^10 words, through shared memory.  With i =
+// (a, m, b), 5 high bits a and 5 low bits b, word (a, m, b) goes to (rev b, rev
+// m, rev a): the 32 x 32 words of one middle part m, 32 rows of 128 contiguous
+// bytes, become those of rev m.  A block moves tile m, and in place tile rev m
+// with it (the block of the smaller of the two), so every sector is read and
+// written whole, once; word by word each 4-byte access moves a 32-byte sector.
+// Bound by HBM: four columns of 2^20 in place 81 -> 7 us, 37 columns of 2^19 out
+// of place 131 -> 34 us, against the word swaps.
+__global__ void __launch_bounds__(256) bit_reverse_tiles_kernel(FftCols t, uint32_t log_n) {
+  __shared__ uint32_t tile[2][32][33];
+  const uint32_t* src = t.src[blockIdx.y];
+  uint32_t* dst = t.dst[blockIdx.y];
+  const bool in_place = src == dst;
+  const uint32_t mid = log_n - 10, m = blockIdx.x, rm = mid ? __brev(m) >> (32 - mid) : 0;
+  if (in_place && m > rm) return;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool both = in_place && m != rm;
+#pragma unroll
+  for (uint32_t u = 0; u < 4; u++) {
+    const uint32_t a = warp + 8 * u;
+    const uint64_t at = ((uint64_t)a << (log_n - 5)) + lane;
+    tile[0][a][lane] = src[at + ((uint64_t)m << 5)];
+    if (both) tile[1][a][lane] = src[at + ((uint64_t)rm << 5)];
+  }
+  __syncthreads();
+  const uint32_t rl = __brev(lane) >> 27;
+#pragma unroll
+  for (uint32_t u = 0; u < 4; u++) {
+    const uint32_t a = warp + 8 * u, ra = __brev(a) >> 27;
+    const uint64_t at = ((uint64_t)a << (log_n - 5)) + lane;
+    dst[at + ((uint64_t)rm << 5)] = tile[0][rl][ra];
+    if (both) dst[at + ((uint64_t)m << 5)] = tile[1][rl][ra];
   }
 }
 
@@ -1426,7 +1448,10 @@ static int bit_reverse_group(const uint32_t* const* src, uint32_t* const* dst, u
       t.src[k] = src[a + k];
       t.dst[k] = dst[a + k];
     }
-    if (lg > 0) {
+    if (lg >= 10) {
+      bit_reverse_tiles_kernel<<<dim3(1u << (lg - 10), nc), 256, 0, s>>>(t, lg);
+      STWO_CHECK_LAUNCH();
+    } else if (lg > 0) {
       const uint64_t n = 1ull << lg;
       const unsigned bx = (unsigned)std::min<uint64_t>((n + 255) / 256, std::max<uint64_t>(1, 148 * 32 / nc));
       bit_reverse_cols_kernel<<<dim3(bx, nc), 256, 0, s>>>(t, lg);
@@ -1870,9 +1895,7 @@ extern "C" int stwo_b200_bit_reverse_column(uint32_t* d_col, uint32_t log_size, 
                                             size_t err_len) {
   STWO_ARG_CHECK(log_size <= 31, "log size %u too large", log_size);
   if (log_size == 0) return ok(err, err_len);
-  uint64_t n = 1ull << log_size;
-  uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 148 * 32);
-  bit_reverse_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(d_col, log_size);
-  STWO_CHECK_LAUNCH();
-  return ok(err, err_len);
+  const uint32_t* src = d_col;
+  int rc = bit_reverse_group(&src, &d_col, 1, log_size, as_stream(stream), err, err_len);
+  return rc ? rc : ok(err, err_len);
 }
