@@ -66,14 +66,7 @@ __device__ __forceinline__ void bfly(uint32_t& a, uint32_t& b, uint32_t t) {
   a = m31_add(a, m);
 }
 
-// Butterflies with the twiddle stored doubled (t2 = 2t < 2^32): the 64-bit
-// product b * t2 has (b t) >> 31 as its high word and 2 (b t mod 2^31) as its
-// low word, so the reduction needs one shift instead of a mask and a funnel
-// shift.  Same (lo, hi) pair, hence the same result, as m31_mul(b, t).
-__device__ __forceinline__ uint32_t m31_mul_tw2(uint32_t b, uint32_t t2) {
-  const uint64_t x = (uint64_t)b * t2;
-  return m31_add((uint32_t)x >> 1, (uint32_t)(x >> 32));
-}
+// Butterflies with the twiddle stored doubled (m31_mul_tw2).
 __device__ __forceinline__ void ibfly2(uint32_t& a, uint32_t& b, uint32_t t2) {
   uint32_t s = m31_add(a, b);
   b = m31_mul_tw2(m31_sub(a, b), t2);

@@ -27,12 +27,14 @@ __host__ __device__ __forceinline__ uint32_t m31_neg(uint32_t a) {
   uint32_t c = M31_P - a;
   return c >= M31_P ? c - M31_P : c;
 }
-__host__ __device__ __forceinline__ uint32_t m31_mul(uint32_t a, uint32_t b) {
-  uint64_t x = (uint64_t)a * b;
-  uint32_t lo = (uint32_t)x & M31_P;
-  uint32_t hi = (uint32_t)(x >> 31);
-  return m31_add(lo, hi);
+// b t with t doubled (t2 = 2t < 2^32): the 64-bit product b * t2 has (b t) >> 31
+// as its high word and 2 (b t mod 2^31) as its low word, so the 31-bit halves
+// come apart with one shift instead of a mask and a funnel shift.
+__host__ __device__ __forceinline__ uint32_t m31_mul_tw2(uint32_t b, uint32_t t2) {
+  const uint64_t x = (uint64_t)b * t2;
+  return m31_add((uint32_t)x >> 1, (uint32_t)(x >> 32));
 }
+__host__ __device__ __forceinline__ uint32_t m31_mul(uint32_t a, uint32_t b) { return m31_mul_tw2(a, b << 1); }
 __host__ __device__ __forceinline__ uint32_t m31_sqr(uint32_t a) { return m31_mul(a, a); }
 __host__ __device__ inline uint32_t m31_pow(uint32_t a, uint64_t e) {
   uint32_t r = 1;
@@ -43,7 +45,23 @@ __host__ __device__ inline uint32_t m31_pow(uint32_t a, uint64_t e) {
   }
   return r;
 }
-__host__ __device__ inline uint32_t m31_inv(uint32_t a) { return m31_pow(a, (uint64_t)M31_P - 2); }
+template <int N>
+__host__ __device__ __forceinline__ uint32_t m31_sqr_n(uint32_t a) {
+  for (int i = 0; i < N; i++) a = m31_sqr(a);
+  return a;
+}
+// a^(P - 2) by an addition chain on P - 2 = 128 (2^24 - 1) + 125: 30 squarings
+// and 7 products in place of the 30 squarings and 29 products of m31_pow, all
+// of them one dependent chain in the row kernels' epilogues.  0 -> 0.
+__host__ __device__ inline uint32_t m31_inv(uint32_t a) {
+  const uint32_t e5 = m31_mul(m31_sqr_n<2>(a), a);
+  const uint32_t e15 = m31_mul(m31_sqr(e5), e5);
+  const uint32_t e125 = m31_mul(m31_sqr_n<3>(e15), e5);
+  const uint32_t e255 = m31_mul(m31_sqr(e125), e5);
+  const uint32_t e16 = m31_mul(m31_sqr_n<8>(e255), e255);  // 2^16 - 1
+  const uint32_t e24 = m31_mul(m31_sqr_n<8>(e16), e255);   // 2^24 - 1
+  return m31_mul(m31_sqr_n<7>(e24), e125);
+}
 // M31::reduce of a u32 (core/fields/m31.rs:58-60 restricted to 32-bit input).
 __host__ __device__ __forceinline__ uint32_t m31_reduce_u32(uint32_t v) {
   uint32_t r = (v & M31_P) + (v >> 31);
