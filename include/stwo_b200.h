@@ -67,6 +67,8 @@ int stwo_b200_memcpy_d2d(void* d_dst, const void* d_src, size_t bytes, void* str
 int stwo_b200_memset(void* d_dst, int value, size_t bytes, void* stream, char* err, size_t err_len);
 int stwo_b200_stream_create(void** stream_out, char* err, size_t err_len);
 int stwo_b200_stream_destroy(void* stream, char* err, size_t err_len);
+/* Waits for the stream.  STWO_B200_ETIMEOUT (once) when a bounded device wait
+ * of an operation enqueued before has given up; its outputs are incomplete. */
 int stwo_b200_stream_sync(void* stream, char* err, size_t err_len);
 /* Pinned host memory for the e2e copies. */
 int stwo_b200_host_alloc(size_t bytes, void** h_out, char* err, size_t err_len);
@@ -480,12 +482,12 @@ int stwo_b200_prover_phase_times(stwo_b200_prover* prover, double* ms_out, uint3
                                  size_t err_len);
 
 /* Wait bound of the prover's column-streaming kernels (composition,
- * quotients): a consumer warp polls a stage's mbarrier at most `polls` times
- * before it gives up, sets the prover's error flag and leaves; the prove then
- * returns STWO_B200_ETIMEOUT.  0 gives up at the first wait (every such
- * prove fails); STWO_B200_STREAM_SPIN_DEFAULT restores the default.  The
- * producer's own waits, including its wait for copies still in flight before
- * its block exits, keep the default bound.  No reference counterpart: this
+ * quotients): a thread polls the mbarrier of its block's tensor-core products
+ * at most `polls` times before it gives up, sets the prover's error flag and
+ * stores nothing more; the prove then returns STWO_B200_ETIMEOUT.  0 gives up
+ * at the first wait (every such prove fails); STWO_B200_STREAM_SPIN_DEFAULT
+ * restores the default.  The wait for products still in flight before such a
+ * block exits keeps the default bound.  No reference counterpart: this
  * exercises the failure path of the bounded device waits. */
 #define STWO_B200_STREAM_SPIN_DEFAULT (1u << 22)
 int stwo_b200_prover_set_stream_spin(stwo_b200_prover* prover, uint32_t polls, char* err, size_t err_len);

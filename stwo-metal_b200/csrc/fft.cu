@@ -22,7 +22,7 @@
 #include "common.cuh"
 #include "fft.hpp"
 #include "field.cuh"
-#include "stream.cuh"
+#include "mbar.cuh"
 
 namespace stwo_b200 {
 

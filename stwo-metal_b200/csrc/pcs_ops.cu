@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "field.cuh"
 #include "pcs.hpp"
+#include "rowdot.cuh"
 #include "rowops.cuh"
 
 namespace stwo_b200 {
@@ -87,6 +88,37 @@ __global__ void __launch_bounds__(256) numerators_kernel(NumeratorTerms t, uint3
       out.c[3][i + r] = v.d;
     }
   }
+}
+
+// The same sums on the tensor cores (rowdot.cuh): whole 512-row tiles, columns
+// and outputs 16-byte aligned.
+__global__ void __launch_bounds__(kDotThreads, kDotBlocks) numerators_dot_kernel(NumeratorTerms t, uint32_t n_terms,
+                                                                       qm31 b_sum, uint64_t n, int accumulate,
+                                                                       Col4 out, uint32_t* err) {
+  extern __shared__ __align__(1024) uint8_t sm8[];
+  const NumeratorTerms* tp = &t;
+  row_dot(
+      sm8, n_terms, (uint32_t)(n >> kDotTileBits), kStreamSpin, err, [=](uint32_t k) { return tp->col[k]; },
+      [=](uint32_t k) { return tp->c[k]; }, []() {}, [](int, uint32_t x) { return x; },
+      [&](uint32_t tile, const qm31(&s)[4]) {
+        const uint64_t i = ((uint64_t)tile << kDotTileBits) + 4 * threadIdx.x;
+        qm31 v[4];
+        if (accumulate) {
+          uint4 o[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) o[k] = *reinterpret_cast<const uint4*>(out.c[k] + i);
+#pragma unroll
+          for (int r = 0; r < 4; r++)
+            v[r] = qm31_add(qm31{u4get(o[0], r), u4get(o[1], r), u4get(o[2], r), u4get(o[3], r)}, s[r]);
+        } else {
+#pragma unroll
+          for (int r = 0; r < 4; r++) v[r] = qm31_sub(s[r], b_sum);
+        }
+        *reinterpret_cast<uint4*>(out.c[0] + i) = make_uint4(v[0].a, v[1].a, v[2].a, v[3].a);
+        *reinterpret_cast<uint4*>(out.c[1] + i) = make_uint4(v[0].b, v[1].b, v[2].b, v[3].b);
+        *reinterpret_cast<uint4*>(out.c[2] + i) = make_uint4(v[0].c, v[1].c, v[2].c, v[3].c);
+        *reinterpret_cast<uint4*>(out.c[3] + i) = make_uint4(v[0].d, v[1].d, v[2].d, v[3].d);
+      });
 }
 
 // ------------------------------------------------- lift_and_accumulate -----
@@ -299,7 +331,14 @@ extern "C" int stwo_b200_accumulate_numerators(const uint32_t* const* d_cols, ui
         aligned = aligned && reinterpret_cast<uintptr_t>(t.col[k]) % 16 == 0;
       }
       const int acc = k0 > 0 ? 1 : 0;
-      if (aligned)
+      bool dot = aligned && n % kDotRows == 0 && nt > 0;
+      for (int k = 0; k < 4; k++) dot = dot && reinterpret_cast<uintptr_t>(out.c[k]) % 16 == 0;
+      if (dot) {
+        static std::atomic<uint32_t> attr{0};
+        STWO_CUDA_TRY(ensure_smem_limit(numerators_dot_kernel, (int)dot_smem(kNumTerms), attr));
+        numerators_dot_kernel<<<dot_grid(dot_smem(nt), 0, (uint32_t)(n >> kDotTileBits)),
+                                kDotThreads, dot_smem(nt), s>>>(t, nt, b_sum, n, acc, out, fault_word());
+      } else if (aligned)
         numerators_kernel<true><<<grid_rows(n / 4, 256), 256, 0, s>>>(t, nt, b_sum, n, acc, out);
       else
         numerators_kernel<false><<<grid_rows(n, 256), 256, 0, s>>>(t, nt, b_sum, n, acc, out);
@@ -441,7 +480,7 @@ extern "C" int stwo_b200_batch_eval_at_point(const uint32_t* const* d_coeffs, ui
   int rc = launch_eval_weights(z, lg, w_lo, w_hi, s, err, err_len);
   for (uint32_t p0 = 0; rc == 0 && p0 < n_polys; p0 += kMaxPolys) {
     const uint32_t np = std::min<uint32_t>(kMaxPolys, n_polys - p0);
-    rc = launch_poly_eval(d_coeffs + p0, np, lg, w_lo, w_hi, partial, vals + p0, s, err, err_len);
+    rc = launch_poly_eval(d_coeffs + p0, np, lg, w_lo, w_hi, partial, vals + p0, fault_word(), s, err, err_len);
   }
   if (rc == 0) {
     const cudaError_t e = cudaMemcpyAsync(values_out, vals, (size_t)n_polys * sizeof(qm31), cudaMemcpyDeviceToHost, s);
@@ -450,6 +489,7 @@ extern "C" int stwo_b200_batch_eval_at_point(const uint32_t* const* d_coeffs, ui
   cudaFreeAsync(scratch, s);
   if (rc) return rc;
   STWO_CUDA_TRY(cudaStreamSynchronize(s));
+  if (take_fault()) return set_err(err, err_len, STWO_B200_ETIMEOUT, "a tensor-core product did not complete in time");
   return ok(err, err_len);
 }
 

@@ -20,9 +20,10 @@
 #include "common.cuh"
 #include "fft.hpp"
 #include "field.cuh"
+#include "mbar.cuh"
 #include "pcs.hpp"
+#include "rowdot.cuh"
 #include "rowops.cuh"
-#include "stream.cuh"
 
 namespace stwo_b200 {
 
@@ -57,8 +58,8 @@ __global__ void wide_fib_trace_kernel(const uint32_t* __restrict__ a, const uint
 // reversed), times the vanishing inverse of the point's trace-coset class.
 // Four consecutive points per thread: 16-byte loads keep four times the bytes
 // in flight per load, which this memory-latency-bound loop needs.
-// n_points % 4 == 0, columns 16-byte aligned.  The streaming form
-// composition_tma_kernel takes every domain of at least one 512-row tile.
+// n_points % 4 == 0, columns 16-byte aligned.  The tensor-core form
+// composition_dot_kernel takes every domain of at least one 512-row tile.
 __global__ void __launch_bounds__(256) composition4_kernel(const uint32_t* __restrict__ evals, uint64_t col_stride,
                                                           uint32_t n_cons, const qm31* __restrict__ powers,
                                                           const uint32_t* __restrict__ denom_inv, uint32_t log_n,
@@ -279,7 +280,8 @@ uint32_t poly_eval_chunks(uint32_t lg) { return lg > 10 ? 1u << (lg - 10) : 1u; 
 uint32_t poly_eval_lo_bits(uint32_t lg) { return lg >= 13 && lg <= 24 ? kEvalLoBits : lg / 2; }
 
 int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg, const qm31* d_w_lo,
-                     const qm31* d_w_hi, qm31* d_partial, qm31* d_out, cudaStream_t s, char* err, size_t err_len) {
+                     const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, cudaStream_t s, char* err,
+                     size_t err_len) {
   STWO_ARG_CHECK(n_polys >= 1 && n_polys <= (uint32_t)kMaxPolys && lg <= 30, "poly eval: bad shape");
   PolyTable pt;
   for (uint32_t c = 0; c < n_polys; c++) pt.p[c] = polys[c];
@@ -319,13 +321,13 @@ struct QuotientParams {
   cpoint init;           // first point of the half coset
   cpoint step_pow[31];   // step * 2^b
   uint32_t log_size;     // lifting domain
-  cpoint tile_pts[256];  // m * step * 2^(log_size - tile bits), m < rows/4 (quotient_tma_kernel)
+  cpoint tile_pts[256];  // m * step * 2^(log_size - tile bits), m < rows/4 (quotient_dot_kernel)
 };
 
 // FRI quotients, 4 consecutive rows per thread: 16-byte column loads and one
 // shared inversion for the four denominators (their norms are inverted
 // together with Montgomery's trick; exact, so equal to four cm31_inv).
-// n % 4 == 0, columns 16-byte aligned.  The streaming form quotient_tma_kernel
+// n % 4 == 0, columns 16-byte aligned.  The tensor-core form quotient_dot_kernel
 // takes every domain of at least two 512-row tiles.
 __device__ __forceinline__ cpoint quotient_point(const QuotientParams& q, uint64_t i) {
   const uint64_t n = 1ull << q.log_size, half = n >> 1;
@@ -411,95 +413,46 @@ __global__ void __launch_bounds__(256) quotient4_kernel(QuotientParams q, PolyTa
   }
 }
 
-// ---- TMA column-streaming versions ----
-// A block owns kStreamRows consecutive rows; consumer thread t owns rows 4t ..
-// 4t+3.  Columns arrive kStreamG at a time through the shared-memory stages of
-// ColumnPipe (cp.async.bulk issued by a producer warp, full/empty mbarriers),
-// so the DRAM reads of the next groups overlap the arithmetic of the current
-// one and no block barrier is taken per group.  Same arithmetic per point as
-// composition4_kernel / quotient4_kernel.
-constexpr int kStreamTileBits = 9, kStreamRows = 1 << kStreamTileBits, kStreamG = 6, kStreamS = 3;
-static_assert(kStreamG == 6, "the fold positions of the streaming kernels assume 6-column groups");
-constexpr int kStreamThreads = kStreamRows / 4;      // consumers: four rows per thread
-constexpr int kStreamBlock = kStreamThreads + 32;    // plus the producer warp
-using StreamPipe = ColumnPipe<kStreamG, kStreamS, kStreamRows, kStreamThreads>;
-constexpr int kPipeBarWords = 2 * kStreamS + (kStreamS * kPipeHeaderWords + 1 + 1) / 2;  // uint64 slots
-constexpr uint32_t kStreamErrWord = 8;  // word of the prover's flag buffer set by a timed-out stage
-constexpr size_t kStreamRing = (size_t)kStreamS * kStreamG * kStreamRows * sizeof(uint32_t);
-constexpr uint32_t kStreamMaxW = 1024;  // QM31 weights staged in shared memory
-constexpr size_t kStreamSmem = kStreamRing + kStreamMaxW * sizeof(uint4);
+// ---- the row kernels on the tensor cores (rowdot.cuh) ----
+// 512-row tiles, four consecutive rows a thread, the sums over the columns as
+// 8-bit products.  Same values as composition4_kernel / quotient4_kernel.
+constexpr uint32_t kStreamErrWord = 8;  // word of the prover's flag buffer set by a wait that ran out
 
-__device__ __forceinline__ void stage_weights(uint4* sw, const qm31* __restrict__ w, uint32_t n) {
-  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) sw[k] = make_uint4(w[k].a, w[k].b, w[k].c, w[k].d);
-}
-
-__global__ void __launch_bounds__(kStreamBlock) composition_tma_kernel(
+__global__ void __launch_bounds__(kDotThreads, kDotBlocks) composition_dot_kernel(
     const uint32_t* __restrict__ evals, uint64_t col_stride, uint32_t n_cons, const qm31* __restrict__ powers,
     const uint32_t* __restrict__ denom_inv, uint32_t log_n, uint64_t n_points, uint32_t* __restrict__ out,
     uint32_t* err, uint32_t spin) {
-  extern __shared__ __align__(128) uint32_t smem[];
-  __shared__ uint64_t bars[kPipeBarWords];
-  uint4* sw = reinterpret_cast<uint4*>(smem + kStreamRing / sizeof(uint32_t));
-  const uint32_t t4 = threadIdx.x * 4;
-  auto col = [evals, col_stride](uint32_t c) { return evals + (uint64_t)c * col_stride; };
-  StreamPipe pipe(smem, bars, n_cons + 2, (uint32_t)(n_points / kStreamRows), spin);
-  stage_weights(sw, powers, n_cons);
-  __syncthreads();  // the last block barrier: the producer warp leaves the loop below
-  if (threadIdx.x >= kStreamThreads) {
-    if (threadIdx.x == kStreamThreads) pipe.produce(col, [](uint32_t, uint32_t*) {}, err);
-    return;
-  }
-  for (uint32_t t = 0; t < pipe.my_tiles; t++) {
-    uint32_t sa[4] = {0, 0, 0, 0}, sb[4] = {0, 0, 0, 0};
-    acc4 row[4];
+  extern __shared__ __align__(1024) uint8_t sm8[];
+  // of the two columns before: the square of the first, P minus that of the second
+  uint32_t sq[4], neg[4];
+  row_dot(
+      sm8, n_cons + 2, (uint32_t)(n_points >> kDotTileBits), spin, err,
+      [=](uint32_t c) { return evals + (uint64_t)c * col_stride; },
+      // column c carries constraint c - 2
+      [=](uint32_t c) { return c >= 2 ? powers[c - 2] : qm31_zero(); },
+      [&]() {
 #pragma unroll
-    for (int r = 0; r < 4; r++) row[r] = {0, 0, 0, 0};
-    // Constraint k = c - 2 of column c = 6g + j: folding after j = 3 in even
-    // groups and after j = 1 and j = 5 in odd ones leaves at most four
-    // products between folds.
-    for (uint32_t g = 0; g < pipe.n_groups; g++) {
-      const uint32_t gg = t * pipe.n_groups + g;
-      if (!pipe.wait(gg, err)) return;
-      const uint32_t nc = pipe.cols_in(g);
-#pragma unroll
-      for (int j = 0; j < kStreamG; j++) {
-        if ((uint32_t)j < nc) {
-          const uint32_t c = g * kStreamG + j;
-          const uint4 v = *reinterpret_cast<const uint4*>(pipe.seg(gg, j) + t4);
-          if (c >= 2) {
-            const uint4 pw4 = sw[c - 2];
-            const qm31 pw{pw4.x, pw4.y, pw4.z, pw4.w};
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-              const uint32_t x = u4get(v, r);
-              acc4_mad(row[r], pw, m31_sub(x, m31_add(sa[r], sb[r])));
-              sa[r] = sb[r];
-              sb[r] = m31_sqr(x);
-            }
-          } else {
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-              sa[r] = sb[r];
-              sb[r] = m31_sqr(u4get(v, r));
-            }
-          }
+        for (int r = 0; r < 4; r++) {
+          sq[r] = 0;
+          neg[r] = M31_P;
         }
-        if ((g & 1) ? (j == 1 || j == 5) : (j == 3)) {
+      },
+      [&](int r, uint32_t x) {
+        const uint32_t w = m31_sub(x, sq[r]) + neg[r];  // <= 2P
+        sq[r] = M31_P - neg[r];
+        neg[r] = M31_P - m31_mul_tw2(x, x << 1);
+        return w;
+      },
+      [&](uint32_t tile, const qm31(&s)[4]) {
+        const uint64_t i = ((uint64_t)tile << kDotTileBits) + 4 * threadIdx.x;
+        qm31 v[4];
 #pragma unroll
-          for (int r = 0; r < 4; r++) acc4_fold(row[r]);
-        }
-      }
-      pipe.release(gg);
-    }
-    const uint64_t i = pipe.tile_row0(t) + t4;
-    qm31 v[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) v[r] = qm31_mul_m31(acc4_reduce(row[r]), __ldg(denom_inv + ((i + r) >> log_n)));
-    *reinterpret_cast<uint4*>(out + i) = make_uint4(v[0].a, v[1].a, v[2].a, v[3].a);
-    *reinterpret_cast<uint4*>(out + n_points + i) = make_uint4(v[0].b, v[1].b, v[2].b, v[3].b);
-    *reinterpret_cast<uint4*>(out + 2 * n_points + i) = make_uint4(v[0].c, v[1].c, v[2].c, v[3].c);
-    *reinterpret_cast<uint4*>(out + 3 * n_points + i) = make_uint4(v[0].d, v[1].d, v[2].d, v[3].d);
-  }
+        for (int r = 0; r < 4; r++) v[r] = qm31_mul_m31(s[r], __ldg(denom_inv + ((i + r) >> log_n)));
+        *reinterpret_cast<uint4*>(out + i) = make_uint4(v[0].a, v[1].a, v[2].a, v[3].a);
+        *reinterpret_cast<uint4*>(out + n_points + i) = make_uint4(v[0].b, v[1].b, v[2].b, v[3].b);
+        *reinterpret_cast<uint4*>(out + 2 * n_points + i) = make_uint4(v[0].c, v[1].c, v[2].c, v[3].c);
+        *reinterpret_cast<uint4*>(out + 3 * n_points + i) = make_uint4(v[0].d, v[1].d, v[2].d, v[3].d);
+      });
 }
 
 // Rows 4t .. 4t+3 of a tile (R = 2^b rows, t < R/4): with r0 a multiple of
@@ -508,107 +461,77 @@ __global__ void __launch_bounds__(kStreamBlock) composition_tma_kernel(
 // bitrev_{b-2}(t) * 2^(log-b) and that + 2^(log-2)); e = 1, 3 are their
 // conjugates in the upper half.  So the two points are B +
 // tile_pts[bitrev_{b-2}(t)] and that + step * 2^(log-2), B = init + J0 * step.
-__global__ void __launch_bounds__(kStreamBlock) quotient_tma_kernel(QuotientParams q, PolyTable cols,
-                                                                   uint32_t n_cols,
-                                                                   const qm31* __restrict__ alpha_pows,
-                                                                   const QuotientDyn* __restrict__ dyn,
-                                                                   uint32_t* __restrict__ out, uint32_t* err,
-                                                                   uint32_t spin) {
+// Bit k of the tile's number is bit log-1-b-k of J0: B is the sum of one entry
+// of each of two tables over 7 bits of it, built by the block, and of the
+// steps of its bits above 14 (domains above 2^23).  A third table would keep a
+// third block off the SM (100 columns: 75 KB of shared memory each).
+constexpr uint32_t kTileTabBits = 7, kTileTabs = 2;
+static_assert((1 << kTileTabBits) == kDotThreads, "thread e builds entry e of each table");
+__global__ void __launch_bounds__(kDotThreads, kDotBlocks) quotient_dot_kernel(QuotientParams q, PolyTable cols,
+                                                                     uint32_t n_cols,
+                                                                     const qm31* __restrict__ alpha_pows,
+                                                                     const QuotientDyn* __restrict__ dyn,
+                                                                     uint32_t* __restrict__ out, uint32_t* err,
+                                                                     uint32_t spin) {
   const QuotientDyn& qd = *dyn;  // read at the epilogue, through the read-only cache
-  extern __shared__ __align__(128) uint32_t smem[];
-  __shared__ uint64_t bars[kPipeBarWords];
-  uint4* sw = reinterpret_cast<uint4*>(smem + kStreamRing / sizeof(uint32_t));
+  extern __shared__ __align__(1024) uint8_t sm8[];
+  __shared__ cpoint tab[kTileTabs][1 << kTileTabBits];
   const uint64_t n = 1ull << q.log_size;
-  const uint32_t t4 = threadIdx.x * 4;
-  const PolyTable* tab = &cols;
-  auto col = [tab](uint32_t c) { return tab->p[c]; };
-  StreamPipe pipe(smem, bars, n_cols, (uint32_t)(n / kStreamRows), spin);
-  stage_weights(sw, alpha_pows, n_cols);
-  __syncthreads();  // the last block barrier: the producer warp leaves the loop below
-  if (threadIdx.x >= kStreamThreads) {
-    if (threadIdx.x == kStreamThreads) {
-      // Tile header: B = init + J0 * step, J0 the bit-reversed first row.
-      const QuotientParams* qp = &q;
-      pipe.produce(col,
-                   [qp, &pipe](uint32_t t, uint32_t* h) {
-                     const uint64_t J0 = __brevll(pipe.tile_row0(t)) >> (64 - qp->log_size);
-                     cpoint b = qp->init;
-                     for (uint32_t k = 0; k + 1 < qp->log_size; k++)
-                       if ((J0 >> k) & 1) b = cpoint_add(b, qp->step_pow[k]);
-                     h[0] = b.x;
-                     h[1] = b.y;
-                   },
-                   err);
-    }
-    return;
+  const uint32_t tile_bits = q.log_size - kDotTileBits;
+#pragma unroll 1
+  for (uint32_t k = 0; k < kTileTabs; k++) {
+    cpoint b = k == 0 ? q.init : cpoint{1, 0};
+    for (uint32_t u = 0; u < kTileTabBits && kTileTabBits * k + u < tile_bits; u++)
+      if ((threadIdx.x >> u) & 1) b = cpoint_add(b, q.step_pow[tile_bits - 1 - kTileTabBits * k - u]);
+    tab[k][threadIdx.x] = b;
   }
-  for (uint32_t t = 0; t < pipe.my_tiles; t++) {
-    const uint64_t r0 = pipe.tile_row0(t);
-    cpoint base{0, 0};
-    acc4 s4[4];
+  // row_dot's first barrier orders the tables before their use
+  const PolyTable* table = &cols;
+  row_dot(
+      sm8, n_cols, 1u << tile_bits, spin, err, [=](uint32_t c) { return table->p[c]; },
+      [=](uint32_t c) { return alpha_pows[c]; }, []() {}, [](int, uint32_t x) { return x; },
+      [&](uint32_t tile, const qm31(&s)[4]) {
+        constexpr uint32_t mask = (1u << kTileTabBits) - 1;
+        cpoint base = tab[0][tile & mask];
+        if (tile_bits > kTileTabBits) base = cpoint_add(base, tab[1][(tile >> kTileTabBits) & mask]);
+        for (uint32_t u = 2 * kTileTabBits; u < tile_bits; u++)
+          if ((tile >> u) & 1) base = cpoint_add(base, q.step_pow[tile_bits - 1 - u]);
+        const cpoint p0 = cpoint_add(base, q.tile_pts[__brev(threadIdx.x) >> (32 - (kDotTileBits - 2))]);
+        const cpoint p2 = cpoint_add(p0, q.step_pow[q.log_size - 2]);
+        const uint32_t xs[4] = {p0.x, p0.x, p2.x, p2.x};
+        const uint32_t ys[4] = {p0.y, m31_neg(p0.y), p2.y, m31_neg(p2.y)};
+        qm31 full[4];
+        cm31 den[4];
+        uint32_t norm[4];
 #pragma unroll
-    for (int r = 0; r < 4; r++) s4[r] = {0, 0, 0, 0};
-    for (uint32_t g = 0; g < pipe.n_groups; g++) {
-      const uint32_t gg = t * pipe.n_groups + g;
-      if (!pipe.wait(gg, err)) return;
-      if (g == 0) {  // header of the tile, valid while this stage is held
-        const uint32_t* h = pipe.head(gg);
-        base = cpoint{h[0], h[1]};
-      }
-      const uint32_t nc = pipe.cols_in(g);
-#pragma unroll
-      for (int j = 0; j < kStreamG; j++) {
-        if ((uint32_t)j < nc) {
-          const uint32_t c = g * kStreamG + j;
-          const uint4 v = *reinterpret_cast<const uint4*>(pipe.seg(gg, j) + t4);
-          const uint4 a4 = sw[c];
-          const qm31 ap{a4.x, a4.y, a4.z, a4.w};
-#pragma unroll
-          for (int r = 0; r < 4; r++) acc4_mad(s4[r], ap, u4get(v, r));
+        for (int r = 0; r < 4; r++) {
+          const qm31 num = qm31_sub(qm31_mul(qd.c, s[r]), qd.B);
+          full[r] = qm31_sub(num, qm31_mul_m31(qd.A, ys[r]));
+          den[r] = cm31_sub(cm31_mul(cm31_sub(qd.prx, cm31{xs[r], 0}), qd.piy),
+                            cm31_mul(cm31_sub(qd.pry, cm31{ys[r], 0}), qd.pix));
+          norm[r] = m31_add(m31_sqr(den[r].a), m31_sqr(den[r].b));
         }
-        if ((g & 1) ? (j == 1 || j == 5) : (j == 3)) {  // at most four products between folds
+        // Montgomery batch inversion of the four norms.
+        const uint32_t p01 = m31_mul(norm[0], norm[1]);
+        const uint32_t p012 = m31_mul(p01, norm[2]);
+        uint32_t inv = m31_inv(m31_mul(p012, norm[3]));
+        uint32_t ninv[4];
+        ninv[3] = m31_mul(inv, p012);
+        inv = m31_mul(inv, norm[3]);
+        ninv[2] = m31_mul(inv, p01);
+        inv = m31_mul(inv, norm[2]);
+        ninv[1] = m31_mul(inv, norm[0]);
+        ninv[0] = m31_mul(inv, norm[1]);
+        qm31 v[4];
 #pragma unroll
-          for (int r = 0; r < 4; r++) acc4_fold(s4[r]);
-        }
-      }
-      pipe.release(gg);
-    }
-    const cpoint p0 = cpoint_add(base, q.tile_pts[__brev(threadIdx.x) >> (32 - (kStreamTileBits - 2))]);
-    const cpoint p2 = cpoint_add(p0, q.step_pow[q.log_size - 2]);
-    const uint32_t xs[4] = {p0.x, p0.x, p2.x, p2.x};
-    const uint32_t ys[4] = {p0.y, m31_neg(p0.y), p2.y, m31_neg(p2.y)};
-    qm31 full[4];
-    cm31 den[4];
-    uint32_t norm[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const qm31 num = qm31_sub(qm31_mul(qd.c, acc4_reduce(s4[r])), qd.B);
-      full[r] = qm31_sub(num, qm31_mul_m31(qd.A, ys[r]));
-      den[r] = cm31_sub(cm31_mul(cm31_sub(qd.prx, cm31{xs[r], 0}), qd.piy),
-                        cm31_mul(cm31_sub(qd.pry, cm31{ys[r], 0}), qd.pix));
-      norm[r] = m31_add(m31_sqr(den[r].a), m31_sqr(den[r].b));
-    }
-    // Montgomery batch inversion of the four norms.
-    const uint32_t p01 = m31_mul(norm[0], norm[1]);
-    const uint32_t p012 = m31_mul(p01, norm[2]);
-    uint32_t inv = m31_inv(m31_mul(p012, norm[3]));
-    uint32_t ninv[4];
-    ninv[3] = m31_mul(inv, p012);
-    inv = m31_mul(inv, norm[3]);
-    ninv[2] = m31_mul(inv, p01);
-    inv = m31_mul(inv, norm[2]);
-    ninv[1] = m31_mul(inv, norm[0]);
-    ninv[0] = m31_mul(inv, norm[1]);
-    qm31 v[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-      v[r] = qm31_mul_cm31(full[r], cm31_mul({den[r].a, m31_neg(den[r].b)}, {ninv[r], 0}));
-    const uint64_t i = r0 + t4;
-    *reinterpret_cast<uint4*>(out + i) = make_uint4(v[0].a, v[1].a, v[2].a, v[3].a);
-    *reinterpret_cast<uint4*>(out + n + i) = make_uint4(v[0].b, v[1].b, v[2].b, v[3].b);
-    *reinterpret_cast<uint4*>(out + 2 * n + i) = make_uint4(v[0].c, v[1].c, v[2].c, v[3].c);
-    *reinterpret_cast<uint4*>(out + 3 * n + i) = make_uint4(v[0].d, v[1].d, v[2].d, v[3].d);
-  }
+        for (int r = 0; r < 4; r++)
+          v[r] = qm31_mul_cm31(full[r], cm31_mul({den[r].a, m31_neg(den[r].b)}, {ninv[r], 0}));
+        const uint64_t i = ((uint64_t)tile << kDotTileBits) + 4 * threadIdx.x;
+        *reinterpret_cast<uint4*>(out + i) = make_uint4(v[0].a, v[1].a, v[2].a, v[3].a);
+        *reinterpret_cast<uint4*>(out + n + i) = make_uint4(v[0].b, v[1].b, v[2].b, v[3].b);
+        *reinterpret_cast<uint4*>(out + 2 * n + i) = make_uint4(v[0].c, v[1].c, v[2].c, v[3].c);
+        *reinterpret_cast<uint4*>(out + 3 * n + i) = make_uint4(v[0].d, v[1].d, v[2].d, v[3].d);
+      });
 }
 
 // Proof-of-work search over nonces (hi << 32) | (low_base + t)
@@ -1426,19 +1349,6 @@ __global__ void __launch_bounds__(kFriTailThreads, 1) fri_tail_kernel(FriTail t,
   }
 }
 
-// Persistent grid of the column-streaming kernels: as many blocks as are
-// resident at once (occupancy of this kernel with its shared memory), never
-// more blocks than tiles.
-template <typename K>
-static unsigned stream_grid(K kernel, size_t smem, uint32_t n_tiles) {
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kStreamBlock, smem);
-  const uint32_t resident = (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, per_sm);
-  return std::max(1u, std::min(n_tiles, resident));
-}
-
 static unsigned grid1d(uint64_t n, unsigned threads) {
   uint64_t b = (n + threads - 1) / threads;
   return (unsigned)std::min<uint64_t>(std::max<uint64_t>(b, 1), 148ull * 32);
@@ -1726,9 +1636,9 @@ class WideFibProver {
       STWO_CUDA_TRY(cudaFuncSetAttribute(tree_top_channel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kFriTailSmem));
       STWO_CUDA_TRY(
-          cudaFuncSetAttribute(composition_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem));
+          cudaFuncSetAttribute(composition_dot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dot_smem(kDotMaxCols)));
       STWO_CUDA_TRY(
-          cudaFuncSetAttribute(quotient_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem));
+          cudaFuncSetAttribute(quotient_dot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dot_smem(kDotMaxCols)));
     }
     log_n = c.log_n_rows;
     N = N_cap = c.n_cols;
@@ -2118,13 +2028,11 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     comp_stride = 1ull << eval_log;
   }
   const uint64_t n_eval = 1ull << eval_log;
-  if (n_eval % kStreamRows == 0 && n_cons <= kStreamMaxW && comp_stride % 4 == 0 &&
+  if (n_eval % kDotRows == 0 && N <= kDotMaxCols && comp_stride % 4 == 0 &&
       reinterpret_cast<uintptr_t>(comp_src) % 16 == 0)
-    composition_tma_kernel<<<stream_grid(composition_tma_kernel, kStreamRing + n_cons * sizeof(uint4),
-                                         (uint32_t)(n_eval / kStreamRows)),
-                             kStreamBlock, kStreamRing + n_cons * sizeof(uint4), s>>>(
-        comp_src, comp_stride, n_cons, d_small, d_denom, log_n, n_eval, d_comp, d_found + kStreamErrWord,
-        stream_spin);
+    composition_dot_kernel<<<dot_grid(dot_smem(N), 0, (uint32_t)(n_eval / kDotRows)), kDotThreads,
+                             dot_smem(N), s>>>(comp_src, comp_stride, n_cons, d_small, d_denom, log_n, n_eval, d_comp,
+                                               d_found + kStreamErrWord, stream_spin);
   else if (n_eval % 4 == 0 && comp_stride % 4 == 0 && reinterpret_cast<uintptr_t>(comp_src) % 16 == 0)
     composition4_kernel<<<grid1d(n_eval / 4, 256), 256, 0, s>>>(comp_src, comp_stride, n_cons, d_small, d_denom,
                                                                 log_n, n_eval, d_comp);
@@ -2170,8 +2078,8 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     std::vector<const uint32_t*> polys(coeff_ptrs.begin(), coeff_ptrs.begin() + N);
     for (int k = 0; k < 8; k++) polys.push_back(split[k]);
     d_vals = d_small + n_w;
-    if ((rc = launch_poly_eval(polys.data(), np, lg, d_small, d_small + (1u << h), d_oods_partial, d_vals, s, err,
-                               err_len)))
+    if ((rc = launch_poly_eval(polys.data(), np, lg, d_small, d_small + (1u << h), d_oods_partial, d_vals,
+                               d_found + kStreamErrWord, s, err, err_len)))
       return rc;
   }
 
@@ -2195,16 +2103,15 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     for (int k = 0; k < 8; k++) cols.p[N + k] = lde[k];
     bool aligned = lift >= 2;
     for (uint32_t c = 0; c < nq; c++) aligned = aligned && reinterpret_cast<uintptr_t>(cols.p[c]) % 16 == 0;
-    if (aligned && lift >= (uint32_t)kStreamTileBits + 1 && nq <= kStreamMaxW) {
-      cpoint g = qp.step_pow[lift - kStreamTileBits], acc = {1, 0};
-      for (int m = 0; m < kStreamRows / 4; m++) {
+    if (aligned && lift >= (uint32_t)kDotTileBits + 1 && nq <= kDotMaxCols) {
+      cpoint g = qp.step_pow[lift - kDotTileBits], acc = {1, 0};
+      for (int m = 0; m < kDotRows / 4; m++) {
         qp.tile_pts[m] = acc;
         acc = cpoint_add(acc, g);
       }
-      quotient_tma_kernel<<<stream_grid(quotient_tma_kernel, kStreamRing + nq * sizeof(uint4),
-                                        (uint32_t)((1ull << lift) / kStreamRows)),
-                            kStreamBlock, kStreamRing + nq * sizeof(uint4), s>>>(
-          qp, cols, nq, d_ap, d_qdyn, d_quot, d_found + kStreamErrWord, stream_spin);
+      quotient_dot_kernel<<<dot_grid(dot_smem(nq), kTileTabs * sizeof(cpoint) << kTileTabBits, (uint32_t)((1ull << lift) / kDotRows)),
+                            kDotThreads, dot_smem(nq), s>>>(qp, cols, nq, d_ap, d_qdyn, d_quot,
+                                                            d_found + kStreamErrWord, stream_spin);
     } else if (aligned) {
       quotient4_kernel<<<grid1d(1ull << (lift - 2), 256), 256, 0, s>>>(qp, cols, nq, d_ap, d_qdyn, d_quot);
     } else {  // pool-allocated columns are 256-byte aligned and lift >= 5
