@@ -274,22 +274,160 @@ __global__ void __launch_bounds__(256, 2) poly_eval_bucket_kernel(PolyTable t, u
   if (lane == 0) partial[unit] = tot;
 }
 
+// The same sums for many polynomials on the tensor cores: up to 128 polynomials
+// are the rows of an 8-bit product (umma.cuh) whose depth is the bucket,
+// D[p][4 k + j] = sum_(e, b) byte_b(c_(p, 1024 beta + e)) byte_j(w_lo[e]_k 2^(8b)
+// mod P).  A polynomial's coefficients are consecutive words, so its row is
+// copied as it lies in memory, 512 bytes (128 coefficients) a step, by 16-byte
+// cp.async into four swizzled operands; a step is copied while the one before
+// it is multiplied.  The block
+// holds the bucket's weights as operand (64 KB) and walks every gridDim.x-th
+// bucket of one group of 128 polynomials; thread p < 128 multiplies
+// polynomial p's bucket sum by w_hi and adds it up, partial[p * gridDim.x +
+// blockIdx.x] in the end.  No multiply-add is left per coefficient: what
+// bounds it is the memory time of the coefficients.
+constexpr uint32_t kEvalStep = 128;                              // coefficients of a step
+constexpr uint32_t kEvalPerBucket = (1u << kEvalLoBits) / kEvalStep;  // steps of a bucket
+constexpr uint32_t kEvalBuf = 4 * kUmmaOperand;                  // bytes of a step's operands
+struct EvalSync {
+  uint64_t bar[2];
+  uint64_t drain;
+  uint32_t tmem;
+  uint32_t pad;
+};
+constexpr size_t kEvalDotSmem = ((1u << kEvalLoBits) / 32) * kDotStage + 2 * kEvalBuf + sizeof(EvalSync);
+__global__ void __launch_bounds__(256, 1) poly_eval_dot_kernel(PolyTable t, uint32_t n_polys, uint32_t n_buckets,
+                                                               const qm31* __restrict__ w_lo,
+                                                               const qm31* __restrict__ w_hi,
+                                                               qm31* __restrict__ partial, uint32_t* err) {
+  extern __shared__ __align__(1024) uint8_t sm8[];
+  uint8_t* opB = sm8;
+  uint8_t* opA = sm8 + ((1u << kEvalLoBits) / 32) * kDotStage;
+  EvalSync* sy = reinterpret_cast<EvalSync*>(opA + 2 * kEvalBuf);
+  const uint32_t tid = threadIdx.x;
+  const uint32_t p0 = blockIdx.y * 128, np = min(128u, n_polys - p0);
+  const uint32_t my_buckets = (n_buckets - blockIdx.x + gridDim.x - 1) / gridDim.x;  // gridDim.x <= n_buckets
+  const uint32_t total = my_buckets * kEvalPerBucket;
+  // step g: thread (warp, lane) copies chunk `lane` of the 512 bytes of rows warp + 8 u
+  const uint32_t warp = tid >> 5, lane = tid & 31;
+  auto fill = [&](uint32_t g) {
+    if (g < total) {
+      const uint64_t at = ((uint64_t)(blockIdx.x + (g / kEvalPerBucket) * gridDim.x) << kEvalLoBits) +
+                          kEvalStep * (g % kEvalPerBucket) + 4 * lane;
+      uint8_t* dst = opA + (g & 1) * kEvalBuf + (lane >> 3) * kUmmaOperand;
+#pragma unroll
+      for (uint32_t u = 0; u < 16; u++) {
+        const uint32_t r = warp + 8 * u;
+        if (r < np)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(dst + sw128(r, 16 * (lane & 7)))),
+                       "l"(t.p[p0 + r] + at)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  if (tid < 32) tmem_alloc<32>(&sy->tmem);
+  if (tid == 0) {
+    mbar_init(&sy->bar[0], 1);
+    mbar_init(&sy->bar[1], 1);
+    mbar_init(&sy->drain, 1);
+    mbar_fence_init();
+  }
+  fill(0);
+  fill(1);
+  for (uint32_t e = tid; e < (1u << kEvalLoBits); e += 256) {
+    const qm31 w = w_lo[e];
+    const uint32_t comp[4] = {w.a, w.b, w.c, w.d};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      uint32_t plane[4];
+      umma_weight(comp[k], plane);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        *reinterpret_cast<uint32_t*>(opB + (e >> 5) * kDotStage + sw128(4 * k + j, 4 * (e & 31))) = plane[j];
+    }
+  }
+  qm31 tot = qm31_zero();
+  bool ok = true;
+  for (uint32_t g = 0; g < total; g++) {
+    const uint32_t in_bucket = g % kEvalPerBucket, bucket = g / kEvalPerBucket;
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // step g has landed, step g + 1 may be in flight
+    umma_fence_operand();
+    umma_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      umma_fence_after();
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const uint64_t a = umma_desc(smem_addr(opA) + (g & 1) * kEvalBuf + u * kUmmaOperand);
+        const uint64_t b = umma_desc(smem_addr(opB) + (4 * in_bucket + u) * kDotStage);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          umma_mma(sy->tmem + kDotCols * (bucket & 1), a + 2 * k, b + 2 * k, umma_idesc(kDotCols),
+                   (in_bucket | u | k) != 0);
+      }
+      umma_commit(&sy->bar[g & 1]);
+    }
+    ok = ok && mbar_wait(&sy->bar[g & 1], (g >> 1) & 1);
+    fill(g + 2);
+    if (in_bucket + 1 == kEvalPerBucket && tid < 128) {
+      umma_fence_after();
+      uint32_t d[16];
+      tmem_ld16(sy->tmem + kDotCols * (bucket & 1) + ((tid & 96) << 16), d);
+      tmem_ld_wait(d);
+      tot = qm31_add(tot, qm31_mul(qm31{umma_value(d), umma_value(d + 4), umma_value(d + 8), umma_value(d + 12)}, w_hi[blockIdx.x + bucket * gridDim.x]));
+    }
+  }
+  if (tid < np && ok) partial[(uint64_t)(p0 + tid) * gridDim.x + blockIdx.x] = tot;
+  if (!ok) {
+    if (tid == 0) {
+      umma_commit(&sy->drain);
+      (void)mbar_wait(&sy->drain, 0);
+    }
+    if (err) *err = 1;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  umma_fence_before();
+  __syncthreads();
+  if (tid < 32) tmem_free<32>(sy->tmem);
+}
+
 uint32_t poly_eval_chunks(uint32_t lg) { return lg > 10 ? 1u << (lg - 10) : 1u; }  // kOodsChunk indices each
 // kEvalLoBits wherever the bucketed form applies (at least kEvalUnitBuckets
 // buckets per polynomial and a w_hi table of at most 2^14 entries).
 uint32_t poly_eval_lo_bits(uint32_t lg) { return lg >= 13 && lg <= 24 ? kEvalLoBits : lg / 2; }
 
+// From 32 polynomials up the tensor-core form (its cost is that of a whole group
+// of 128): 108 polynomials of 2^20 119 -> 82 us.  Below, most of a product's
+// rows would be empty.
+constexpr uint32_t kEvalDotPolys = 32;
 int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg, const qm31* d_w_lo,
                      const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, cudaStream_t s, char* err,
                      size_t err_len) {
   STWO_ARG_CHECK(n_polys >= 1 && n_polys <= (uint32_t)kMaxPolys && lg <= 30, "poly eval: bad shape");
   PolyTable pt;
-  for (uint32_t c = 0; c < n_polys; c++) pt.p[c] = polys[c];
+  bool aligned = true;  // for 16-byte loads; other pointers take the chunked form
+  for (uint32_t c = 0; c < n_polys; c++) {
+    pt.p[c] = polys[c];
+    aligned = aligned && reinterpret_cast<uintptr_t>(polys[c]) % 16 == 0;
+  }
   const uint32_t h = poly_eval_lo_bits(lg);
-  if (h == kEvalLoBits) {
+  if (h == kEvalLoBits && aligned) {
     // 2^(lg - h) >= kEvalUnitBuckets buckets of 1024 indices per polynomial
     const uint32_t units_per_poly = (1u << (lg - h)) / kEvalUnitBuckets;
     const uint32_t units = n_polys * units_per_poly;
+    if (n_polys >= kEvalDotPolys) {
+      static std::atomic<uint32_t> attr{0};
+      STWO_CUDA_TRY(ensure_smem_limit(poly_eval_dot_kernel, (int)kEvalDotSmem, attr));
+      const uint32_t groups = (n_polys + 127) / 128, buckets = 1u << (lg - h);
+      const uint32_t blocks = std::min(buckets, std::max(1u, 148u / groups));
+      poly_eval_dot_kernel<<<dim3(blocks, groups), 256, kEvalDotSmem, s>>>(pt, n_polys, buckets, d_w_lo, d_w_hi,
+                                                                           d_partial, fault);
+      STWO_CHECK_LAUNCH();
+      oods_reduce_kernel<<<n_polys, 256, 0, s>>>(d_partial, blocks, d_out);
+      STWO_CHECK_LAUNCH();
+      return STWO_B200_OK;
+    }
     poly_eval_bucket_kernel<<<(units + 7) / 8, 256, 0, s>>>(pt, n_polys, units_per_poly, d_w_lo, d_w_hi, d_partial);
     STWO_CHECK_LAUNCH();
     oods_reduce_kernel<<<n_polys, 256, 0, s>>>(d_partial, units_per_poly, d_out);

@@ -60,3 +60,19 @@ def test_numerators_alignment(oracle, in_off, out_off):
     ref, _ = oracle.accumulate_numerators(cols, log_n, point, terms)
     for o, r in zip(outs, ref):
         assert (o.buf.to_host()[out_off:] == r).all()
+
+
+@pytest.mark.parametrize("log_n", [12, 13, 14, 17])
+@pytest.mark.parametrize("n_polys", [1, 31, 32, 33, 127, 128, 129, 300])
+def test_batch_eval_groups(oracle, log_n, n_polys):
+    # 2^12 takes the chunked kernel, from 2^13 up 32 polynomials or more the tensor cores
+    rng = np.random.default_rng(1000 * log_n + n_polys)
+    polys = [words(rng, 1 << log_n) for _ in range(min(n_polys, 9))]
+    polys[0][:] = P
+    dev = [DeviceColumn.from_host(p) for p in polys]
+    point = rng.integers(1, P, 8, dtype=np.uint32)
+    got = B200Backend().batch_eval_at_point([dev[k % len(dev)] for k in range(n_polys)], point)
+    want = [B200Backend().eval_at_point(d, point) for d in dev]  # the integer-pipe kernels
+    for k in range(n_polys):
+        assert (got[k] == want[k % len(dev)]).all(), k
+    assert (want[1 % len(dev)] == oracle.eval_at_secure_point(polys[1 % len(dev)], point)).all()
