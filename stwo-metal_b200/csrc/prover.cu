@@ -714,6 +714,32 @@ __global__ void gather_kernel(const uint64_t* __restrict__ addrs, uint32_t n, ui
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = *reinterpret_cast<const uint32_t*>(addrs[i]);
 }
+// Copies up to kMaxSegments word ranges of device memory into one page-locked
+// host buffer, a block each: the host's view of a phase in one launch of about
+// 3 us, where a stream copy of a few bytes takes 6 us (3 of them between copies)
+// and a proof reads 20 to 40 of them.
+constexpr int kMaxSegments = 48;
+struct Segments {
+  const uint32_t* src[kMaxSegments];
+  uint32_t at[kMaxSegments];     // word of the host buffer
+  uint32_t words[kMaxSegments];
+  uint32_t n = 0;
+  // Takes `bytes` (a multiple of 4) at byte `at_byte` of the host buffer.
+  bool add(const void* p, size_t at_byte, size_t bytes) {
+    if (n == kMaxSegments) return false;
+    src[n] = reinterpret_cast<const uint32_t*>(p);
+    at[n] = (uint32_t)(at_byte / 4);
+    words[n] = (uint32_t)(bytes / 4);
+    n++;
+    return true;
+  }
+};
+__global__ void __launch_bounds__(256) download_kernel(Segments g, uint32_t* __restrict__ host) {
+  const uint32_t* src = g.src[blockIdx.x];
+  const uint32_t at = g.at[blockIdx.x], n = g.words[blockIdx.x];
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) host[at + i] = src[i];
+}
+
 // 32-byte hashes at 32-byte aligned addresses (Merkle tree nodes).
 __global__ void gather_hashes_kernel(const uint64_t* __restrict__ addrs, uint32_t n, uint4* __restrict__ out) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -821,8 +847,10 @@ __device__ void dev_chan_mix_staged(DevChannel* ch, const uint32_t* s_words, uin
 constexpr uint32_t kFinishMaxLast = 64;
 __global__ void fri_finish_kernel(const DevChannel* __restrict__ ch, const uint32_t* __restrict__ last,
                                   uint32_t last_log, uint32_t bound_log, const uint32_t* __restrict__ xi,
-                                  uint32_t n_inv, uint32_t pow_bits, uint32_t* __restrict__ pow) {
+                                  uint32_t n_inv, uint32_t pow_bits, uint32_t* __restrict__ pow,
+                                  uint32_t* __restrict__ found) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  *found = 0xFFFFFFFFu;  // no nonce yet
   const uint32_t n = 1u << last_log;
   qm31 v[kFinishMaxLast];
   for (uint32_t i = 0; i < n; i++) {
@@ -962,6 +990,14 @@ __device__ qm31 qm31_pow_u32(qm31 x, uint32_t e) {
     e >>= 1;
   }
   return r;
+}
+
+// The device channel's state and the cleared error word of a proof.
+__global__ void proof_begin_kernel(DevChannel init, DevChannel* ch, uint32_t* flag) {
+  if (threadIdx.x == 0) {
+    *ch = init;
+    *flag = 0;
+  }
 }
 
 // ---- device-side Fiat-Shamir steps before the FRI commit ----
@@ -1691,8 +1727,6 @@ class WideFibProver {
   std::vector<uint32_t> words_buf;
   qm31* d_oods_partial = nullptr;  // OODS partial sums (polynomials x chunks)
   qm31* h_pinned = nullptr;       // staging for small uploads / downloads
-  DevChannel* h_chan = nullptr;   // staging of the device channel state (own region: the
-                                  // quotient upload from h_pinned may still be in flight)
   size_t h_pinned_bytes = 0;
   uint8_t* h_tx = nullptr;          // pre-FRI transcript download: roots 1-2, FsOut, sampled values
   size_t h_tx_bytes = 0;
@@ -1740,7 +1774,6 @@ class WideFibProver {
     for (void* p : allocs) cudaFree(p);  // empty in measure mode
     if (h_pinned) cudaFreeHost(h_pinned);
     if (h_tx) cudaFreeHost(h_tx);
-    if (h_chan) cudaFreeHost(h_chan);
     if (s) cudaStreamDestroy(s);
   }
 
@@ -1847,10 +1880,9 @@ class WideFibProver {
     if ((rc = alloc((void**)&d_alphas, (fri.size() + 2) * sizeof(qm31), err, err_len))) return rc;
     if ((rc = alloc((void**)&d_fs, sizeof(FsOut), err, err_len))) return rc;
     if ((rc = alloc((void**)&d_qdyn, sizeof(QuotientDyn), err, err_len))) return rc;
-    h_pinned_bytes = std::max<size_t>(small_q * sizeof(qm31), (16ull << last_log) + 65536);
+    h_pinned_bytes = std::max<size_t>(small_q * sizeof(qm31), (16ull << last_log) + (1u << 18));
     if (measure) return 0;
     STWO_CUDA_TRY(cudaMallocHost((void**)&h_pinned, h_pinned_bytes));
-    STWO_CUDA_TRY(cudaMallocHost((void**)&h_chan, sizeof(DevChannel)));
     h_tx_bytes = 64 + sizeof(FsOut) + (size_t)(N + 8) * sizeof(qm31) + 16;  // + the stream error word
     STWO_CUDA_TRY(cudaMallocHost((void**)&h_tx, h_tx_bytes));
     {
@@ -2078,7 +2110,6 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
   HostChannel ch(m31);
   int rc;
   const uint64_t rows = 1ull << log_n;
-  STWO_CUDA_TRY(cudaMemsetAsync(d_found + kStreamErrWord, 0, 4, s));
   // ---- tree 0: empty preprocessed trace -> Blake2s("") ----
   Hash32 root0;
   {
@@ -2089,12 +2120,12 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
   // The device channel carries the transcript from here to the end of the
   // FRI commit; the host replays it after one download.
   {
-    DevChannel* hc = h_chan;
-    std::memset(hc, 0, sizeof(DevChannel));
-    std::memcpy(hc->digest, ch.digest().data(), 32);
-    hc->n_draws = ch.n_draws();
-    hc->m31 = m31 ? 1 : 0;
-    STWO_CUDA_TRY(cudaMemcpyAsync(d_chan, hc, sizeof(DevChannel), cudaMemcpyHostToDevice, s));
+    DevChannel hc{};
+    std::memcpy(hc.digest, ch.digest().data(), 32);
+    hc.n_draws = ch.n_draws();
+    hc.m31 = m31 ? 1 : 0;
+    proof_begin_kernel<<<1, 32, 0, s>>>(hc, d_chan, d_found + kStreamErrWord);
+    STWO_CHECK_LAUNCH();
   }
 
   // ---- tree 1: trace ----
@@ -2266,12 +2297,17 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
   const uint32_t last_log = cfg.log_last_layer_degree_bound + blowup;
   // Download of the pre-FRI transcript values, so that the host replays
   // them while the device runs the FRI commit.
-  STWO_CUDA_TRY(cudaMemcpyAsync(h_tx, t1.layer(0), 32, cudaMemcpyDeviceToHost, s));
-  STWO_CUDA_TRY(cudaMemcpyAsync(h_tx + 32, t2.layer(0), 32, cudaMemcpyDeviceToHost, s));
-  STWO_CUDA_TRY(cudaMemcpyAsync(h_tx + 64, d_fs, sizeof(FsOut), cudaMemcpyDeviceToHost, s));
-  STWO_CUDA_TRY(cudaMemcpyAsync(h_tx + 64 + sizeof(FsOut), d_vals, np * sizeof(qm31), cudaMemcpyDeviceToHost, s));
   const size_t tx_flag_off = 64 + sizeof(FsOut) + np * sizeof(qm31);
-  STWO_CUDA_TRY(cudaMemcpyAsync(h_tx + tx_flag_off, d_found + kStreamErrWord, 4, cudaMemcpyDeviceToHost, s));
+  {
+    Segments g;
+    g.add(t1.layer(0), 0, 32);
+    g.add(t2.layer(0), 32, 32);
+    g.add(d_fs, 64, sizeof(FsOut));
+    g.add(d_vals, 64 + sizeof(FsOut), np * sizeof(qm31));
+    g.add(d_found + kStreamErrWord, tx_flag_off, 4);
+    download_kernel<<<g.n, 256, 0, s>>>(g, reinterpret_cast<uint32_t*>(h_tx));
+    STWO_CHECK_LAUNCH();
+  }
   STWO_CUDA_TRY(cudaEventRecord(ev_tx, s));
   if ((rc = run_fri(err, err_len))) return rc;
   if (dev_finish) {
@@ -2280,9 +2316,8 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     // own and continues the search from the second batch when this one
     // finds no nonce
     fri_finish_kernel<<<1, 32, 0, s>>>(d_chan, d_last, last_log, cfg.log_last_layer_degree_bound, d_last_xi,
-                                       last_n_inv, cfg.pow_bits, d_pow);
+                                       last_n_inv, cfg.pow_bits, d_pow, d_found);
     STWO_CHECK_LAUNCH();
-    STWO_CUDA_TRY(cudaMemsetAsync(d_found, 0xFF, 4, s));
     grind_dev_kernel<<<kGrindBatch / 256, 256, 0, s>>>(d_pow, 0, 0, cfg.pow_bits, m31, d_found);
     STWO_CHECK_LAUNCH();
   }
@@ -2360,32 +2395,33 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
   uint32_t fri_end_draws = 0;
   std::vector<qm31> dev_alphas;
   {
-    uint8_t* hpw = reinterpret_cast<uint8_t*>(h_pinned);
     size_t off = 0;
-    STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, tq.layer(0), 32, cudaMemcpyDeviceToHost, s));
+    Segments g;
+    bool fits = g.add(tq.layer(0), off, 32);
     off += 32;
     for (auto& l : fri) {
-      STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, l.tree.layer(0), 32, cudaMemcpyDeviceToHost, s));
+      fits = fits && g.add(l.tree.layer(0), off, 32);
       off += 32;
     }
     alpha_off = off;
-    STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, d_alphas, (fri.size() + 1) * sizeof(qm31), cudaMemcpyDeviceToHost, s));
+    fits = fits && g.add(d_alphas, off, (fri.size() + 1) * sizeof(qm31));
     off += (fri.size() + 1) * sizeof(qm31);
     chan_off = off;
-    STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, d_chan, sizeof(DevChannel), cudaMemcpyDeviceToHost, s));
+    fits = fits && g.add(d_chan, off, sizeof(DevChannel));
     off += sizeof(DevChannel);
     flag_off = off;
-    STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, d_found + kStreamErrWord, 4, cudaMemcpyDeviceToHost, s));
+    fits = fits && g.add(d_found + kStreamErrWord, off, 4);
     off += 16;
     if (dev_finish) {
       pow_off = off;
-      STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, d_pow, 36, cudaMemcpyDeviceToHost, s));
-      STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off + 48, d_found, 4, cudaMemcpyDeviceToHost, s));
+      fits = fits && g.add(d_pow, off, 36) && g.add(d_found, off + 48, 4);
       off += 64;
     }
     last_off = off;
-    STWO_ARG_CHECK(off + 16 * n_last <= h_pinned_bytes, "pinned staging too small for the last layer");
-    STWO_CUDA_TRY(cudaMemcpyAsync(hpw + off, d_last, 16 * n_last, cudaMemcpyDeviceToHost, s));
+    fits = fits && g.add(d_last, off, 16 * n_last);
+    STWO_ARG_CHECK(fits && off + 16 * n_last <= h_pinned_bytes, "pinned staging too small for the last layer");
+    download_kernel<<<g.n, 256, 0, s>>>(g, reinterpret_cast<uint32_t*>(h_pinned));
+    STWO_CHECK_LAUNCH();
     STWO_CUDA_TRY(cudaStreamSynchronize(s));
     const DevChannel* dc = reinterpret_cast<const DevChannel*>(hp + chan_off);
     // A timed-out stream leaves the transcript built on partial rows, so its
@@ -2581,34 +2617,48 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
   TreeDecommit& td2 = td_buf[1];
   plan_tree(td1, eval_ptrs, L1, t1);
   plan_tree(td2, lde, L2, t2);
-  if ((rc = ensure_gather(g.addrs.size(), err, err_len))) return rc;
   {
     size_t n = g.addrs.size();
-    std::vector<uint32_t>& words = words_buf;
-    words.resize(n);
-    // upload addresses through the pinned staging buffer in chunks
-    size_t chunk = h_pinned_bytes / 8;
-    for (size_t off = 0; off < n; off += chunk) {
-      size_t m = std::min(chunk, n - off);
-      std::memcpy(h_pinned, g.addrs.data() + off, m * 8);
-      STWO_CUDA_TRY(cudaMemcpyAsync(d_gather_addr + off, h_pinned, m * 8, cudaMemcpyHostToDevice, s));
-      // the staging buffer is reused by the next chunk only; the gather and
-      // the download below are ordered after the upload on the stream
-      if (off + m < n) STWO_CUDA_TRY(cudaStreamSynchronize(s));
-    }
-    gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_gather_addr, (uint32_t)n, d_gather_out);
-    STWO_CHECK_LAUNCH();
-    if (!replayed && (rc = replay_fri())) return rc;
-    size_t wchunk = h_pinned_bytes / 4;
-    for (size_t off = 0; off < n; off += wchunk) {
-      size_t m = std::min(wchunk, n - off);
-      STWO_CUDA_TRY(cudaMemcpyAsync(h_pinned, d_gather_out + off, m * 4, cudaMemcpyDeviceToHost, s));
+    const uint32_t* words = nullptr;
+    if (n * 12 <= h_pinned_bytes) {
+      // the kernel reads the plan from, and writes the words to, page-locked
+      // memory: no copies around it
+      std::memcpy(h_pinned, g.addrs.data(), n * 8);
+      uint32_t* h_words = reinterpret_cast<uint32_t*>(h_pinned) + 2 * n;
+      gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(reinterpret_cast<const uint64_t*>(h_pinned), (uint32_t)n,
+                                                                h_words);
+      STWO_CHECK_LAUNCH();
+      if (!replayed && (rc = replay_fri())) return rc;
       STWO_CUDA_TRY(cudaStreamSynchronize(s));
-      std::memcpy(words.data() + off, h_pinned, m * 4);
+      words = h_words;
+    } else {
+      // longer plans go through the device buffers, staged in chunks
+      if ((rc = ensure_gather(n, err, err_len))) return rc;
+      words_buf.resize(n);
+      size_t chunk = h_pinned_bytes / 8;
+      for (size_t off = 0; off < n; off += chunk) {
+        size_t m = std::min(chunk, n - off);
+        std::memcpy(h_pinned, g.addrs.data() + off, m * 8);
+        STWO_CUDA_TRY(cudaMemcpyAsync(d_gather_addr + off, h_pinned, m * 8, cudaMemcpyHostToDevice, s));
+        // the staging buffer is reused by the next chunk only; the gather and
+        // the download below are ordered after the upload on the stream
+        if (off + m < n) STWO_CUDA_TRY(cudaStreamSynchronize(s));
+      }
+      gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_gather_addr, (uint32_t)n, d_gather_out);
+      STWO_CHECK_LAUNCH();
+      if (!replayed && (rc = replay_fri())) return rc;
+      size_t wchunk = h_pinned_bytes / 4;
+      for (size_t off = 0; off < n; off += wchunk) {
+        size_t m = std::min(wchunk, n - off);
+        STWO_CUDA_TRY(cudaMemcpyAsync(h_pinned, d_gather_out + off, m * 4, cudaMemcpyDeviceToHost, s));
+        STWO_CUDA_TRY(cudaStreamSynchronize(s));
+        std::memcpy(words_buf.data() + off, h_pinned, m * 4);
+      }
+      words = words_buf.data();
     }
     // ---- serialize (canonical layout, struct field order of
     // core/pcs/quotients.rs:27-35 and core/fri.rs:361-395) ----
-    auto hash_at = [&](size_t slot, ProofOut& o) { o.h(reinterpret_cast<const uint8_t*>(words.data() + slot)); };
+    auto hash_at = [&](size_t slot, ProofOut& o) { o.h(reinterpret_cast<const uint8_t*>(words + slot)); };
     const char magic[8] = {'S', 'T', 'W', 'O', 'P', 'R', 'F', '1'};
     if (out.bytes.capacity() < last_proof_bytes) out.bytes.reserve(last_proof_bytes);
     out.bytes.assign(magic, magic + 8);
@@ -2951,8 +3001,6 @@ struct SeededFriProver {
     const size_t nw = word_addr.size(), nh = hash_addr.size(), total = nw + nh;
     if (total > gather_cap) {
       const size_t cap = std::max<size_t>(total * 2, 4096);
-      if ((rc = alloc((void**)&d_gather_addr, cap * 8, err, err_len))) return rc;
-      if ((rc = alloc((void**)&d_gather_out, cap * 32, err, err_len))) return rc;
       if (h_stage) cudaFreeHost(h_stage);
       h_stage = nullptr;
       STWO_CUDA_TRY(cudaMallocHost((void**)&h_stage, cap * 40));
@@ -2961,16 +3009,14 @@ struct SeededFriProver {
     uint64_t* h_addr = reinterpret_cast<uint64_t*>(h_stage);
     std::memcpy(h_addr, word_addr.data(), nw * 8);
     std::memcpy(h_addr + nw, hash_addr.data(), nh * 8);
-    STWO_CUDA_TRY(cudaMemcpyAsync(d_gather_addr, h_addr, total * 8, cudaMemcpyHostToDevice, s));
-    uint32_t* d_words = reinterpret_cast<uint32_t*>(d_gather_out);
-    uint4* d_hashes = reinterpret_cast<uint4*>(d_gather_out + ((nw * 4 + 31) / 32) * 32);
-    gather_kernel<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(d_gather_addr, (uint32_t)nw, d_words);
-    STWO_CHECK_LAUNCH();
-    gather_hashes_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(d_gather_addr + nw, (uint32_t)nh, d_hashes);
-    STWO_CHECK_LAUNCH();
+    // plan and results in page-locked memory, read and written by the kernels
     uint8_t* h_out = h_stage + gather_cap * 8;
-    const size_t out_bytes = ((nw * 4 + 31) / 32) * 32 + nh * 32;
-    STWO_CUDA_TRY(cudaMemcpyAsync(h_out, d_gather_out, out_bytes, cudaMemcpyDeviceToHost, s));
+    uint32_t* h_words = reinterpret_cast<uint32_t*>(h_out);
+    uint4* h_hashes = reinterpret_cast<uint4*>(h_out + ((nw * 4 + 31) / 32) * 32);
+    gather_kernel<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(h_addr, (uint32_t)nw, h_words);
+    STWO_CHECK_LAUNCH();
+    gather_hashes_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(h_addr + nw, (uint32_t)nh, h_hashes);
+    STWO_CHECK_LAUNCH();
     STWO_CUDA_TRY(cudaStreamSynchronize(s));
     const uint32_t* words = reinterpret_cast<const uint32_t*>(h_out);
     const uint8_t* hashes = h_out + ((nw * 4 + 31) / 32) * 32;
