@@ -26,7 +26,9 @@
 #include <deque>
 #include <list>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -143,6 +145,10 @@ struct Server {
   void worker() {
     cudaSetDevice(device);
     char err[512];
+    // Where every proof of this worker is written first: not cleared, and only
+    // the pages that a proof reaches are ever touched (a cleared buffer of this
+    // size for each request took longer than a proof of 2^14 rows).
+    std::unique_ptr<uint8_t[]> proof(new (std::nothrow) uint8_t[kMaxProofBytes]);
     for (;;) {
       Request* r = nullptr;
       Resident* res = nullptr;
@@ -177,11 +183,11 @@ struct Server {
       if (!rc) rc = stwo_b200_memcpy_h2d(res->d_a, r->a.data(), nb, res->stream, err, sizeof(err));
       if (!rc) rc = stwo_b200_memcpy_h2d(res->d_b, r->b.data(), nb, res->stream, err, sizeof(err));
       size_t len = 0;
+      if (!rc && !proof) rc = set_err(err, sizeof(err), STWO_B200_ENOMEM, "no host memory for the proof");
       if (!rc) {
-        r->proof.resize(kMaxProofBytes);
-        rc = stwo_b200_prove_wide_fib_cols(res->prover, r->cfg.n_cols, res->d_a, res->d_b, r->proof.data(),
-                                           r->proof.size(), &len, err, sizeof(err));
-        r->proof.resize(rc ? 0 : len);
+        rc = stwo_b200_prove_wide_fib_cols(res->prover, r->cfg.n_cols, res->d_a, res->d_b, proof.get(),
+                                           kMaxProofBytes, &len, err, sizeof(err));
+        if (!rc) r->proof.assign(proof.get(), proof.get() + len);
       }
       std::lock_guard<std::mutex> lk(mu);
       r->rc = rc;

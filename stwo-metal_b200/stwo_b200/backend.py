@@ -94,6 +94,45 @@ class DeviceColumn(DeviceBuffer):
         return self.download(np.uint32, self.length)
 
 
+# Buffers up to this size that belong together (the coordinates of a secure
+# column, the top of a tree) are parts of one allocation: below it a stream-
+# ordered allocation and its release (3 to 5 us with the calls) cost more than
+# the kernels that fill it.  Above it each stands alone, so that what a caller
+# keeps does not hold what they dropped: a kept part holds 4 MiB at most.
+PART_BYTES = 1 << 20
+
+
+class _Part(DeviceColumn):
+    """A part of a buffer; the buffer is freed with the last of its parts."""
+
+    def __init__(self, owner: DeviceBuffer, offset: int, nbytes: int):
+        self.owner = owner
+        self.nbytes = nbytes
+        self.length = nbytes // 4
+        self.stream = owner.stream
+        self.ptr = owner.ptr + offset
+
+    def close(self):
+        self.ptr = 0
+        self.owner = None
+
+
+def _parts(sizes, stream):
+    """Buffers of these byte sizes, at 256-byte boundaries of one allocation."""
+    at = [0]
+    for b in sizes:
+        at.append(at[-1] + (b + 255) // 256 * 256)
+    owner = DeviceBuffer(at[-1], stream)
+    return [_Part(owner, a, b) for a, b in zip(at, sizes)]
+
+
+def _tree_layers(log_size, stream):
+    """Buffers of 2^k hashes, k = 0..log_size."""
+    top = min(log_size, (PART_BYTES // 32).bit_length() - 1)
+    return (_parts([32 << k for k in range(top + 1)], stream) +
+            [DeviceBuffer(32 << k, stream) for k in range(top + 1, log_size + 1)])
+
+
 class SecureColumn:
     """QM31 column as four M31 coordinate columns (SecureColumnByCoords)."""
 
@@ -107,6 +146,8 @@ class SecureColumn:
 
     @classmethod
     def empty(cls, length, stream=None):
+        if 0 < 4 * length <= PART_BYTES:
+            return cls(_parts([4 * length] * 4, stream))
         return cls([DeviceColumn(length, stream) for _ in range(4)])
 
     def to_host(self):
@@ -237,7 +278,7 @@ class B200Backend:
 
     def build_merkle_layers(self, cols, lifting_log_size: int, m31_output: bool = False):
         """Layers root first: layers[k] holds 2^k hashes."""
-        layers = [DeviceBuffer(32 << k, self.stream) for k in range(lifting_log_size + 1)]
+        layers = _tree_layers(lifting_log_size, self.stream)
         ffi.call("stwo_b200_merkle_build_layers", _ptr_array(cols), _u32_array([c.log_size for c in cols]),
                  C.c_uint32(len(cols)), C.c_uint32(lifting_log_size), C.c_int(int(m31_output)),
                  _ptr_array(layers), self.stream)
@@ -298,14 +339,10 @@ class B200Backend:
         cb = (SampleBatch * max(1, len(batches)))()
         keep, outs = [], []
         for b, (point, terms) in enumerate(batches):
-            arr = (NumeratorTerm * max(1, len(terms)))()
-            for k, (idx, val, alpha) in enumerate(terms):
-                arr[k].column_index = int(idx)
-                arr[k].sample_value = _words(val, 4)
-                arr[k].random_coeff = _words(alpha, 4)
+            arr = _terms(terms)
             keep.append(arr)
             cb[b].point = _words(point, 8)
-            cb[b].terms = C.cast(arr, C.POINTER(NumeratorTerm))
+            cb[b].terms = C.cast(C.c_void_p(arr.ctypes.data), C.POINTER(NumeratorTerm))
             cb[b].n_terms = len(terms)
             outs.append(SecureColumn.empty(1 << log_n, self.stream))
         first = (C.c_uint32 * (4 * max(1, len(batches))))()
@@ -350,7 +387,7 @@ class B200Backend:
         out = (C.c_uint32 * (4 * max(1, len(polys))))()
         ffi.call("stwo_b200_batch_eval_at_point", _ptr_array(polys), C.c_uint32(len(polys)),
                  C.c_uint32(polys[0].log_size if polys else 0), _words(point, 8), out, self.stream)
-        return np.array(out[:4 * len(polys)], np.uint32).reshape(len(polys), 4)
+        return np.frombuffer(out, np.uint32, 4 * len(polys)).copy().reshape(len(polys), 4)
 
     def eval_at_point(self, poly: DeviceColumn, point) -> np.ndarray:
         out = (C.c_uint32 * 4)()
@@ -404,7 +441,25 @@ class AccumulatedNumeratorsC(C.Structure):
 def _words(v, n):
     a = np.asarray(v, dtype=np.uint32).reshape(-1)
     assert a.size == n
-    return (C.c_uint32 * n)(*[int(x) for x in a])
+    return (C.c_uint32 * n)(*a.tolist())
+
+
+def _rows(vals, n):
+    """One row of n words for each value."""
+    if all(type(v) is np.ndarray and v.dtype == np.uint32 and v.size == n for v in vals):
+        return np.concatenate([v.reshape(-1) for v in vals]).reshape(-1, n)
+    return np.array([list(_words(v, n)) for v in vals], np.uint32)
+
+
+def _terms(terms) -> np.ndarray:
+    """(column index, value, random coefficient) terms as NumeratorTerm's 9 words each."""
+    arr = np.zeros((max(1, len(terms)), 9), np.uint32)
+    if terms:
+        index, value, coeff = zip(*terms, strict=True)
+        arr[:, 0] = [int(i) & 0xFFFFFFFF for i in index]
+        arr[:, 1:5] = _rows(value, 4)
+        arr[:, 5:] = _rows(coeff, 4)
+    return arr
 
 
 def layer_to_host(buf: DeviceBuffer) -> np.ndarray:
@@ -450,7 +505,7 @@ class Committer:
         self.lifting_log_size = L.value
 
     def new_layers(self):
-        return [DeviceBuffer(32 << k, self.stream) for k in range(self.lifting_log_size + 1)]
+        return _tree_layers(self.lifting_log_size, self.stream)
 
     def commit(self, evals, coeffs, ldes, layers):
         ffi.call("stwo_b200_committer_commit", self._h, _ptr_array(evals), _ptr_array(coeffs), _ptr_array(ldes),

@@ -49,9 +49,13 @@ def declared_symbols() -> list[str]:
     return sorted(set(re.findall(r"\b(stwo_b200_[a-z0-9_]+)\s*\(", text)))
 
 
+_Message = C.c_char * 512
+_MESSAGE_LEN = C.c_size_t(512)
+
+
 def call(fn_name: str, *args) -> None:
-    err = C.create_string_buffer(512)
-    rc = getattr(load(), fn_name)(*args, err, C.c_size_t(len(err)))
+    err = _Message()
+    rc = getattr(_lib or load(), fn_name)(*args, err, _MESSAGE_LEN)
     if rc != 0:
         raise B200Error(rc, err.value.decode(errors="replace"))
 

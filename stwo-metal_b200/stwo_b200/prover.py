@@ -24,6 +24,13 @@ def wide_fib_config(log_n_rows: int, n_cols: int = 100, log_blowup: int = 1, pow
                          line_fold_step, int(m31_channel))
 
 
+def _proof_buffer(cap: int):
+    """Memory for a proof of at most cap bytes (not cleared: clearing 4 MiB takes
+    longer than a small proof) and its address."""
+    buf = np.empty(cap, np.uint8)
+    return buf, C.c_void_p(buf.ctypes.data)
+
+
 class WideFibProver:
     """Owns the device buffers of one proof shape; proves repeatedly."""
 
@@ -36,30 +43,30 @@ class WideFibProver:
         self.handle = h
 
     def prove(self, a: DeviceColumn, b: DeviceColumn, cap: int = 1 << 22) -> bytes:
-        buf = (C.c_uint8 * cap)()
+        buf, at = _proof_buffer(cap)
         n = C.c_size_t()
-        ffi.call("stwo_b200_prove_wide_fib", self.handle, C.c_void_p(a.ptr), C.c_void_p(b.ptr), buf,
+        ffi.call("stwo_b200_prove_wide_fib", self.handle, C.c_void_p(a.ptr), C.c_void_p(b.ptr), at,
                  C.c_size_t(cap), C.byref(n))
-        return C.string_at(buf, n.value)
+        return buf[:n.value].tobytes()
 
     def prove_cols(self, a: DeviceColumn, b: DeviceColumn, n_cols: int, cap: int = 1 << 22) -> bytes:
         """The proof of an n_cols-wide trace (3 <= n_cols <= the prover's width)."""
-        buf = (C.c_uint8 * cap)()
+        buf, at = _proof_buffer(cap)
         n = C.c_size_t()
         ffi.call("stwo_b200_prove_wide_fib_cols", self.handle, C.c_uint32(n_cols), C.c_void_p(a.ptr),
-                 C.c_void_p(b.ptr), buf, C.c_size_t(cap), C.byref(n))
-        return C.string_at(buf, n.value)
+                 C.c_void_p(b.ptr), at, C.c_size_t(cap), C.byref(n))
+        return buf[:n.value].tobytes()
 
     def prove_host(self, a: np.ndarray, b: np.ndarray, cap: int = 1 << 22) -> bytes:
         """The proof from host columns (numpy, uint32); copied by the prover,
         overlapped with the trace generation when the memory is pinned."""
         a = np.ascontiguousarray(a, dtype=np.uint32)
         b = np.ascontiguousarray(b, dtype=np.uint32)
-        buf = (C.c_uint8 * cap)()
+        buf, at = _proof_buffer(cap)
         n = C.c_size_t()
         ffi.call("stwo_b200_prove_wide_fib_host", self.handle, C.c_void_p(a.ctypes.data), C.c_void_p(b.ctypes.data),
-                 buf, C.c_size_t(cap), C.byref(n))
-        return C.string_at(buf, n.value)
+                 at, C.c_size_t(cap), C.byref(n))
+        return buf[:n.value].tobytes()
 
     def prove_host_into(self, a_ptr: int, b_ptr: int, out_buf, cap: int) -> int:
         """prove_host from raw host pointers (e.g. pinned buffers) into out_buf."""
@@ -171,11 +178,11 @@ class ProveServer:
         return t.value
 
     def wait(self, ticket: int, cap: int = 1 << 22):
-        buf = C.create_string_buffer(cap)
+        buf, at = _proof_buffer(cap)
         n = C.c_size_t()
         times = (C.c_double * 3)()
-        ffi.call("stwo_b200_server_wait", self._h, C.c_uint64(ticket), buf, C.c_size_t(cap), C.byref(n), times)
-        return C.string_at(buf, n.value), {"queued_ms": times[0], "service_ms": times[1], "latency_ms": times[2]}
+        ffi.call("stwo_b200_server_wait", self._h, C.c_uint64(ticket), at, C.c_size_t(cap), C.byref(n), times)
+        return buf[:n.value].tobytes(), {"queued_ms": times[0], "service_ms": times[1], "latency_ms": times[2]}
 
     def stats(self) -> dict:
         st = ServerStats()
