@@ -7,8 +7,8 @@
 // thread per leaf absorbs 16 columns per compression; for every column a warp
 // reads 32 consecutive (or pairwise repeated) words, so loads are coalesced
 // without a shared-memory transpose.  Node layers hash 64-byte child pairs with
-// one final compression (core/vcs_lifted/blake2_merkle.rs:18-25); a block
-// builds up to 8 layers of a subtree in shared memory per launch.
+// one final compression (core/vcs_lifted/blake2_merkle.rs:18-25); the upper
+// levels of a tree are one launch (tree.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -17,6 +17,7 @@
 #include "blake2s.cuh"
 #include "common.cuh"
 #include "field.cuh"
+#include "tree.cuh"
 
 namespace stwo_b200 {
 
@@ -111,74 +112,18 @@ __global__ void __launch_bounds__(256) lifted_leaves_kernel(LeafCols t, uint32_t
   }
 }
 
-// Hashes `levels` consecutive node layers.  Block b hashes `width` parents
-// of `in` (2^in_log hashes) at the first level, keeps them in shared memory
-// and continues up its subtree; every produced layer lv goes to outs[lv].
-struct NodeOuts {
-  uint8_t* out[8];
-};
-
-// LAT selects the shortest-dependency Blake2s form, for launches of a few
-// blocks where one compression's latency (not throughput) sets the time.
+// The levels below level in_log of a tree, down to `stop` (tree_climb): a block
+// has 2^kTreeBlockLog hashes of level in_log (all of them where that has fewer).
 template <bool LAT>
-__global__ void __launch_bounds__(256) node_layers_kernel(const uint8_t* in, uint32_t in_log, uint32_t levels, int m31,
-                                                         NodeOuts outs) {
-  __shared__ uint32_t buf[2][256 * 8];
-  // level 0: parents of `in`
-  uint64_t parents0 = 1ull << (in_log - 1);
-  uint32_t width = parents0 < 256 ? (uint32_t)parents0 : 256u;  // parents of this block at level 0
-  uint64_t first_parent = (uint64_t)blockIdx.x * width;
-  uint32_t tid = threadIdx.x;
-  int cur = 0;
-  if (tid < width) {
-    uint64_t p = first_parent + tid;
-    const uint4* src = reinterpret_cast<const uint4*>(in + p * 64);
-    uint32_t m[16];
-    uint4 a = src[0], b = src[1], c = src[2], d = src[3];
-    m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
-    m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
-    m[8] = c.x; m[9] = c.y; m[10] = c.z; m[11] = c.w;
-    m[12] = d.x; m[13] = d.y; m[14] = d.z; m[15] = d.w;
-    uint32_t h[8];
-    blake2s_init(h);
-    if (LAT)
-      blake2s_compress_lat(h, m, 64, true);
-    else
-      blake2s_compress(h, m, 64, true);
-    if (m31) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) h[k] = m31_reduce_u32(h[k]);
-    }
-    store_hash(outs.out[0], p, h, false);
-#pragma unroll
-    for (int k = 0; k < 8; k++) buf[cur][tid * 8 + k] = h[k];
-  }
+__global__ void __launch_bounds__(kTreeThreads) node_levels_kernel(const uint8_t* in, uint32_t in_log, uint32_t stop,
+                                                                   int m31, TreeLevels t, uint32_t* arrivals) {
+  __shared__ TreeSmem sm;
+  const uint32_t w = 1u << min(in_log, kTreeBlockLog);
+  const uint64_t base = (uint64_t)blockIdx.x * w;
+  tree_stage(sm.ping, in + base * 32, w);
   __syncthreads();
-  for (uint32_t lv = 1; lv < levels; lv++) {
-    width >>= 1;
-    if (width == 0) break;
-    uint64_t first = first_parent >> lv;
-    if (tid < width) {
-      uint32_t m[16];
-#pragma unroll
-      for (int k = 0; k < 16; k++) m[k] = buf[cur][tid * 16 + k];
-      uint32_t h[8];
-      blake2s_init(h);
-      if (LAT)
-      blake2s_compress_lat(h, m, 64, true);
-    else
-      blake2s_compress(h, m, 64, true);
-      if (m31) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) h[k] = m31_reduce_u32(h[k]);
-      }
-      store_hash(outs.out[lv], first + tid, h, false);
-#pragma unroll
-      for (int k = 0; k < 8; k++) buf[cur ^ 1][tid * 8 + k] = h[k];
-    }
-    cur ^= 1;
-    __syncthreads();
-  }
+  const uint4* root;
+  tree_climb<LAT>(sm, t, in_log, base, w, stop, arrivals, m31 != 0, []() {}, &root);
 }
 
 // Parent hash of the 64-byte child pair in m (throughput form), reduced to
@@ -393,17 +338,20 @@ int build_leaves_impl(const uint32_t* const* d_cols, const uint32_t* log_sizes, 
   return STWO_B200_OK;
 }
 
-constexpr uint32_t kSubtree3MinLog = 19;
+constexpr uint32_t kSubtree3MinLog = 18;
+uint32_t node_levels_wide(uint32_t L) {
+  while (L >= kSubtree3MinLog) L -= 3;
+  return L;
+}
 
 // Builds layers [in_log - 1 .. stop_log] from layer `in` (2^in_log hashes);
 // outs_by_log[k] is the destination of layer log k.
 int build_node_layers_impl(const uint8_t* in, uint32_t in_log, uint32_t stop_log, int m31,
-                           uint8_t* const* outs_by_log, cudaStream_t s, char* err, size_t err_len) {
+                           uint8_t* const* outs_by_log, uint32_t* arrivals, cudaStream_t s, char* err,
+                           size_t err_len) {
   uint32_t cur_log = in_log;
   const uint8_t* cur = in;
   while (cur_log > stop_log) {
-    // Wide layers: three levels per thread while the third level still has
-    // 2^16 parents (256 blocks of 256 threads).
     if (cur_log - stop_log >= 3 && cur_log >= kSubtree3MinLog) {
       const uint64_t n = 1ull << (cur_log - 3);
       node_subtree3_kernel<<<grid_for(n, 256), 256, 0, s>>>(cur, n, m31, outs_by_log[cur_log - 1],
@@ -413,23 +361,46 @@ int build_node_layers_impl(const uint8_t* in, uint32_t in_log, uint32_t stop_log
       cur_log -= 3;
       continue;
     }
-    uint32_t levels = std::min<uint32_t>(8, cur_log - stop_log);
-    uint64_t parents0 = 1ull << (cur_log - 1);
-    uint32_t width = (uint32_t)std::min<uint64_t>(256, parents0);
-    // a block produces width >> (lv) parents at level lv; keep it >= 1
-    while (levels > 1 && (width >> (levels - 1)) == 0) levels--;
-    NodeOuts o;
-    for (uint32_t lv = 0; lv < levels; lv++) o.out[lv] = outs_by_log[cur_log - 1 - lv];
-    unsigned blocks = (unsigned)(parents0 / width);
-    if (blocks <= 148)
-      node_layers_kernel<true><<<blocks, 256, 0, s>>>(cur, cur_log, levels, m31, o);
+    const bool whole = stop_log == 0 && cur_log <= kTreeMaxLog;
+    const uint32_t stop = whole || cur_log - stop_log <= kTreeBlockLog ? stop_log : cur_log - kTreeBlockLog;
+    const unsigned blocks = tree_blocks(cur_log, kTreeBlockLog);
+    TreeLevels t;
+    for (uint32_t k = stop; k < cur_log; k++) t.out[k] = outs_by_log[k];
+    uint32_t* arr = nullptr;
+    if (whole && blocks > 1) {
+      arr = arrivals;
+      if (!arr) {  // the root is written after every block has arrived
+        arr = reinterpret_cast<uint32_t*>(outs_by_log[0]);
+        STWO_CUDA_TRY(cudaMemsetAsync(arr, 0, sizeof(uint32_t), s));
+      }
+    }
+    // The throughput form only where a level of the launch is several warps a
+    // scheduler and there is no chain of levels behind it.
+    if (!whole && blocks > 512)
+      node_levels_kernel<false><<<blocks, kTreeThreads, 0, s>>>(cur, cur_log, stop, m31, t, arr);
     else
-      node_layers_kernel<false><<<blocks, 256, 0, s>>>(cur, cur_log, levels, m31, o);
+      node_levels_kernel<true><<<blocks, kTreeThreads, 0, s>>>(cur, cur_log, stop, m31, t, arr);
     STWO_CHECK_LAUNCH();
-    cur = outs_by_log[cur_log - levels];
-    cur_log -= levels;
+    cur = outs_by_log[stop];
+    cur_log = stop;
   }
   return STWO_B200_OK;
+}
+
+int build_layers_impl(const uint32_t* const* d_cols, const uint32_t* log_sizes, uint32_t n_cols, uint32_t L, int m31,
+                      uint8_t* const* d_layers, uint32_t* arrivals, cudaStream_t s, char* err, size_t err_len) {
+  // prover/vcs_lifted/ops.rs:37 stable sort by length.
+  std::vector<uint32_t> order(n_cols);
+  for (uint32_t i = 0; i < n_cols; i++) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return log_sizes[a] < log_sizes[b]; });
+  std::vector<const uint32_t*> cols(n_cols);
+  std::vector<uint32_t> logs(n_cols);
+  for (uint32_t i = 0; i < n_cols; i++) {
+    cols[i] = d_cols[order[i]];
+    logs[i] = log_sizes[order[i]];
+  }
+  const int rc = build_leaves_impl(cols.data(), logs.data(), n_cols, L, m31, d_layers[L], d_layers, s, err, err_len);
+  return rc ? rc : build_node_layers_impl(d_layers[L], L, 0, m31, d_layers, arrivals, s, err, err_len);
 }
 
 }  // namespace stwo_b200
@@ -450,7 +421,7 @@ extern "C" int stwo_b200_merkle_build_next_layer(const uint8_t* d_prev, uint32_t
   std::vector<uint8_t*> outs(prev_log_size, nullptr);
   outs[prev_log_size - 1] = d_out;
   int rc = build_node_layers_impl(d_prev, prev_log_size, prev_log_size - 1, m31_output, outs.data(),
-                                  as_stream(stream), err, err_len);
+                                  nullptr, as_stream(stream), err, err_len);
   return rc ? rc : ok(err, err_len);
 }
 
@@ -464,20 +435,7 @@ extern "C" int stwo_b200_merkle_build_layers(const uint32_t* const* d_cols, cons
     int rc = build_leaves_impl(nullptr, nullptr, 0, 0, m31_output, d_layers[0], nullptr, s, err, err_len);
     return rc ? rc : ok(err, err_len);
   }
-  // prover/vcs_lifted/ops.rs:37 stable sort by length.
-  std::vector<uint32_t> order(n_cols);
-  for (uint32_t i = 0; i < n_cols; i++) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return log_sizes[a] < log_sizes[b]; });
-  std::vector<const uint32_t*> cols(n_cols);
-  std::vector<uint32_t> logs(n_cols);
-  for (uint32_t i = 0; i < n_cols; i++) {
-    cols[i] = d_cols[order[i]];
-    logs[i] = log_sizes[order[i]];
-  }
-  const uint32_t L = lifting_log_size;
-  int rc = build_leaves_impl(cols.data(), logs.data(), n_cols, L, m31_output, d_layers[L], d_layers, s, err, err_len);
-  if (rc) return rc;
-  rc = build_node_layers_impl(d_layers[L], L, 0, m31_output, d_layers, s, err, err_len);
+  int rc = build_layers_impl(d_cols, log_sizes, n_cols, lifting_log_size, m31_output, d_layers, nullptr, s, err, err_len);
   return rc ? rc : ok(err, err_len);
 }
 
@@ -486,7 +444,7 @@ extern "C" int stwo_b200_merkle_build_nodes(uint8_t* const* d_layers, uint32_t l
   STWO_ARG_CHECK(d_layers != nullptr, "null layers");
   STWO_ARG_CHECK(lifting_log_size <= 31, "bad lifting log size");
   int rc = build_node_layers_impl(d_layers[lifting_log_size], lifting_log_size, 0, m31_output, d_layers,
-                                  as_stream(stream), err, err_len);
+                                  nullptr, as_stream(stream), err, err_len);
   return rc ? rc : ok(err, err_len);
 }
 

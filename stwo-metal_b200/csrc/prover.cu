@@ -24,14 +24,9 @@
 #include "pcs.hpp"
 #include "rowdot.cuh"
 #include "rowops.cuh"
+#include "tree.cuh"
 
 namespace stwo_b200 {
-
-int build_leaves_impl(const uint32_t* const* d_cols, const uint32_t* log_sizes, uint32_t n_cols, uint32_t L,
-                      int m31, uint8_t* d_leaves, uint8_t* const* layer_ws, cudaStream_t s, char* err,
-                      size_t err_len);
-int build_node_layers_impl(const uint8_t* in, uint32_t in_log, uint32_t stop_log, int m31,
-                           uint8_t* const* outs_by_log, cudaStream_t s, char* err, size_t err_len);
 
 // ----------------------------------------------------------------- kernels --
 
@@ -554,6 +549,7 @@ __global__ void __launch_bounds__(256) quotient4_kernel(QuotientParams q, PolyTa
 // ---- the row kernels on the tensor cores (rowdot.cuh) ----
 // 512-row tiles, four consecutive rows a thread, the sums over the columns as
 // 8-bit products.  Same values as composition4_kernel / quotient4_kernel.
+constexpr uint32_t kArrivalsWord = 9;   // word of the same buffer that the tree launches count their blocks in
 constexpr uint32_t kStreamErrWord = 8;  // word of the prover's flag buffer set by a wait that ran out
 
 __global__ void __launch_bounds__(kDotThreads, kDotBlocks) composition_dot_kernel(
@@ -1186,6 +1182,40 @@ __host__ __device__ constexpr uint64_t fold_threads(uint32_t log_out) {
   return log_out > kFoldPairLog ? 1ull << (log_out - 1) : 1ull << log_out;
 }
 
+// Output o of fold_line (prover/backend/cpu/fri.rs:67-92) of 2^log_m values, n_in
+// words a coordinate column.
+__device__ __forceinline__ qm31 fold_line_at(const uint32_t* __restrict__ in, uint64_t n_in, uint32_t log_m,
+                                             uint32_t fold_step, const qm31& a0, const uint32_t* __restrict__ itw,
+                                             uint64_t tw_len, uint64_t o) {
+  if (fold_step == 1) {
+    const uint32_t* lt = itw + (tw_len - (1ull << log_m));
+    const qm31 fx = {__ldg(in + 2 * o), __ldg(in + n_in + 2 * o), __ldg(in + 2 * n_in + 2 * o),
+                     __ldg(in + 3 * n_in + 2 * o)};
+    const qm31 fnx = {__ldg(in + 2 * o + 1), __ldg(in + n_in + 2 * o + 1), __ldg(in + 2 * n_in + 2 * o + 1),
+                      __ldg(in + 3 * n_in + 2 * o + 1)};
+    return qm31_add(qm31_add(fx, fnx), qm31_mul(a0, qm31_mul_m31(qm31_sub(fx, fnx), __ldg(lt + o))));
+  }
+  qm31 v[1 << 6];
+  const uint32_t w = 1u << fold_step;
+  for (uint32_t j = 0; j < w; j++) {
+    const uint64_t i = o * w + j;
+    v[j] = {__ldg(in + i), __ldg(in + n_in + i), __ldg(in + 2 * n_in + i), __ldg(in + 3 * n_in + i)};
+  }
+  qm31 a = a0;
+  for (uint32_t st = 0; st < fold_step; st++) {
+    const uint32_t* lt = itw + (tw_len - (1ull << (log_m - st)));
+    const uint32_t pairs = w >> (st + 1);
+    for (uint32_t j = 0; j < pairs; j++) {
+      const qm31 fx = v[2 * j], fnx = v[2 * j + 1];
+      const qm31 f0 = qm31_add(fx, fnx);
+      const qm31 f1 = qm31_mul_m31(qm31_sub(fx, fnx), __ldg(lt + o * pairs + j));
+      v[j] = qm31_add(f0, qm31_mul(a, f1));
+    }
+    a = qm31_mul(a, a);
+  }
+  return v[0];
+}
+
 // fold_line with alpha read from device memory (prover/backend/cpu/fri.rs:67-92).
 // When `leaves` is not null the fold also writes the leaf hashes of the next
 // layer's tree (its Merkle leaf layer), saving a launch and a re-read.
@@ -1222,46 +1252,13 @@ __global__ void fold_line_dev_kernel(const uint32_t* __restrict__ in, uint32_t l
     }
     return;
   }
-  if (fold_step == 1) {
-    const uint32_t* lt = itw + (tw_len - (1ull << log_m));
-    for (uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; o < n_out;
-         o += (uint64_t)gridDim.x * blockDim.x) {
-      qm31 fx = {__ldg(in + 2 * o), __ldg(in + n_in + 2 * o), __ldg(in + 2 * n_in + 2 * o), __ldg(in + 3 * n_in + 2 * o)};
-      qm31 fnx = {__ldg(in + 2 * o + 1), __ldg(in + n_in + 2 * o + 1), __ldg(in + 2 * n_in + 2 * o + 1),
-                  __ldg(in + 3 * n_in + 2 * o + 1)};
-      qm31 v = qm31_add(qm31_add(fx, fnx), qm31_mul(a0, qm31_mul_m31(qm31_sub(fx, fnx), __ldg(lt + o))));
-      out[o] = v.a;
-      out[n_out + o] = v.b;
-      out[2 * n_out + o] = v.c;
-      out[3 * n_out + o] = v.d;
-      if (leaves) fri_leaf_store(leaves, o, v, m31 != 0);
-    }
-    return;
-  }
   for (uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; o < n_out; o += (uint64_t)gridDim.x * blockDim.x) {
-    qm31 v[1 << 6];
-    const uint32_t w = 1u << fold_step;
-    for (uint32_t j = 0; j < w; j++) {
-      uint64_t i = o * w + j;
-      v[j] = {__ldg(in + i), __ldg(in + n_in + i), __ldg(in + 2 * n_in + i), __ldg(in + 3 * n_in + i)};
-    }
-    qm31 a = a0;
-    for (uint32_t st = 0; st < fold_step; st++) {
-      const uint32_t* lt = itw + (tw_len - (1ull << (log_m - st)));
-      uint32_t pairs = w >> (st + 1);
-      for (uint32_t j = 0; j < pairs; j++) {
-        qm31 fx = v[2 * j], fnx = v[2 * j + 1];
-        qm31 f0 = qm31_add(fx, fnx);
-        qm31 f1 = qm31_mul_m31(qm31_sub(fx, fnx), __ldg(lt + o * pairs + j));
-        v[j] = qm31_add(f0, qm31_mul(a, f1));
-      }
-      a = qm31_mul(a, a);
-    }
-    out[o] = v[0].a;
-    out[n_out + o] = v[0].b;
-    out[2 * n_out + o] = v[0].c;
-    out[3 * n_out + o] = v[0].d;
-    if (leaves) fri_leaf_store(leaves, o, v[0], m31 != 0);
+    const qm31 v = fold_line_at(in, n_in, log_m, fold_step, a0, itw, tw_len, o);
+    out[o] = v.a;
+    out[n_out + o] = v.b;
+    out[2 * n_out + o] = v.c;
+    out[3 * n_out + o] = v.d;
+    if (leaves) fri_leaf_store(leaves, o, v, m31 != 0);
   }
 }
 
@@ -1270,6 +1267,18 @@ __global__ void fold_line_dev_kernel(const uint32_t* __restrict__ in, uint32_t l
 struct Src4 {
   const uint32_t* c[4];  // the four coordinate columns
 };
+// Output i of it.
+__device__ __forceinline__ qm31 fold_circle_at(const Src4& src, const uint32_t* __restrict__ lt0, const qm31& alpha,
+                                               uint64_t i) {
+  const uint32_t b = __ldg(lt0 + ((i >> 1) ^ 1));
+  const uint32_t yinv = ((i ^ (i >> 1)) & 1) ? m31_neg(b) : b;
+  const qm31 fp = {__ldg(src.c[0] + 2 * i), __ldg(src.c[1] + 2 * i), __ldg(src.c[2] + 2 * i), __ldg(src.c[3] + 2 * i)};
+  const qm31 fnp = {__ldg(src.c[0] + 2 * i + 1), __ldg(src.c[1] + 2 * i + 1), __ldg(src.c[2] + 2 * i + 1),
+                    __ldg(src.c[3] + 2 * i + 1)};
+  const qm31 f0 = qm31_add(fp, fnp);
+  const qm31 f1 = qm31_mul_m31(qm31_sub(fp, fnp), yinv);
+  return qm31_add(qm31_zero(), qm31_add(f0, qm31_mul(alpha, f1)));
+}
 __global__ void fold_circle_first_dev_kernel(Src4 src, uint32_t log_n, const qm31* __restrict__ d_alpha,
                                              const uint32_t* __restrict__ itw, uint64_t tw_len,
                                              uint32_t* __restrict__ dst, uint8_t* __restrict__ leaves, int m31) {
@@ -1304,14 +1313,7 @@ __global__ void fold_circle_first_dev_kernel(Src4 src, uint32_t log_n, const qm3
     return;
   }
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_out; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t b = __ldg(lt0 + ((i >> 1) ^ 1));
-    uint32_t yinv = ((i ^ (i >> 1)) & 1) ? m31_neg(b) : b;
-    qm31 fp = {__ldg(src.c[0] + 2 * i), __ldg(src.c[1] + 2 * i), __ldg(src.c[2] + 2 * i), __ldg(src.c[3] + 2 * i)};
-    qm31 fnp = {__ldg(src.c[0] + 2 * i + 1), __ldg(src.c[1] + 2 * i + 1), __ldg(src.c[2] + 2 * i + 1),
-                __ldg(src.c[3] + 2 * i + 1)};
-    qm31 f0 = qm31_add(fp, fnp);
-    qm31 f1 = qm31_mul_m31(qm31_sub(fp, fnp), yinv);
-    qm31 v = qm31_add(qm31_zero(), qm31_add(f0, qm31_mul(alpha, f1)));
+    const qm31 v = fold_circle_at(src, lt0, alpha, i);
     dst[i] = v.a;
     dst[n_out + i] = v.b;
     dst[2 * n_out + i] = v.c;
@@ -1386,55 +1388,83 @@ __device__ const uint4* tree_levels_smem(uint8_t* base, uint32_t lg, uint4* src,
   return src;
 }
 
-// Top of one FRI layer tree and its Fiat-Shamir step: hashes levels
-// top_log-1 .. 0 from tree level top_log (2^top_log hashes in global memory,
-// top_log <= kFriTailLog), then mixes the root and draws alpha.
-__global__ void __launch_bounds__(kFriTailThreads, 1) tree_top_channel_kernel(uint8_t* base, uint32_t top_log,
-                                                                              DevChannel* ch, qm31* alpha,
-                                                                              int m31) {
-  extern __shared__ uint4 tail_smem[];
-  uint4* ping = tail_smem;
-  uint4* pong = tail_smem + (2u << kFriTailLog);
-  const bool m31b = m31 != 0;
-  const uint4* src = ping;
+// The Fiat-Shamir step of a layer behind its tree's root: the channel is
+// loaded before the block's last levels, where the load costs no time.
+struct LayerChannel {
+  DevChannel* ch;
+  qm31* alpha;
   ChanRegs cr;
-  if (threadIdx.x == 0) chan_load(ch, cr);  // used after the tree levels
-  if (top_log == 0) {
-    if (threadIdx.x == 0) {
-      const uint4* r = reinterpret_cast<const uint4*>(base);
-      ping[0] = r[0];
-      ping[1] = r[1];
-    }
-    __syncthreads();
-  } else {
-    const uint32_t np = 1u << (top_log - 1);
-    const uint4* in = reinterpret_cast<const uint4*>(base + (((size_t)1 << top_log) - 1) * 32);
-    for (uint32_t p = threadIdx.x; p < np; p += blockDim.x) {
-      uint32_t m[16];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint4 w = __ldg(in + 4 * p + q);
-        m[4 * q] = w.x;
-        m[4 * q + 1] = w.y;
-        m[4 * q + 2] = w.z;
-        m[4 * q + 3] = w.w;
-      }
-      uint32_t h[8];
-      blake2s_init(h);
-      blake2s_compress_lat(h, m, 64, true);
-      dev_finalize(h, m31b);
-      put_hash(base + ((size_t)np - 1) * 32, ping, p, h);
-    }
-    __syncthreads();
-    src = tree_levels_smem(base, top_log - 1, ping, pong, m31b);
+  __device__ __forceinline__ void begin() {
+    if (threadIdx.x == 0) chan_load(ch, cr);
   }
-  if (threadIdx.x == 0) {
-    const uint4 a = src[0], b = src[1];
-    const uint32_t root[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    chan_mix_root(cr, root);
+  __device__ __forceinline__ void end(const uint4* root) {
+    if (threadIdx.x != 0) return;
+    const uint4 a = root[0], b = root[1];  // slots 0 and 1
+    const uint32_t h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    chan_mix_root(cr, h);
     *alpha = chan_draw_felt(cr);
     chan_store(ch, cr);
   }
+};
+
+// The levels below level in_log of one FRI layer's tree (2^in_log hashes in
+// global memory, in_log <= kTreeMaxLog), then the root's mix and the draw of
+// alpha.
+__global__ void __launch_bounds__(kTreeThreads) fri_nodes_kernel(const uint8_t* in, uint32_t in_log, TreeLevels t,
+                                                                 uint32_t* arrivals, DevChannel* ch, qm31* alpha,
+                                                                 int m31) {
+  __shared__ TreeSmem sm;
+  const uint32_t w = 1u << min(in_log, kTreeBlockLog);
+  const uint64_t base = (uint64_t)blockIdx.x * w;
+  tree_stage(sm.ping, in + base * 32, w);
+  __syncthreads();
+  LayerChannel c{ch, alpha, {}};
+  const uint4* root;
+  if (tree_climb<true>(sm, t, in_log, base, w, 0, gridDim.x > 1 ? arrivals : nullptr, m31 != 0, [&]() { c.begin(); },
+                       &root))
+    c.end(root);
+}
+
+// A whole FRI layer of 2^L values (kFriTailLog < L <= kFriLayerLog): the fold
+// that makes it (of the circle evaluation, or of the layer before it), its
+// leaves, its tree, the root's mix and the draw of its alpha, one value a
+// thread.  Larger layers fold with wide loads and hash several levels a thread
+// first.  Measured against a launch each for the fold, the lower levels and the
+// top with the channel: see enqueue_fri.
+constexpr uint32_t kFriLayerLog = 16;
+static_assert(kFriLayerLog <= kTreeLastLog + 7, "the last block stages one hash for each block of 2^7 values");
+template <bool CIRCLE>
+__global__ void __launch_bounds__(kTreeThreads) fri_layer_kernel(Src4 src, uint32_t log_m, uint32_t fold_step,
+                                                                 const qm31* __restrict__ d_alpha,
+                                                                 const uint32_t* __restrict__ itw, uint64_t tw_len,
+                                                                 uint32_t* __restrict__ out, TreeLevels t,
+                                                                 uint32_t* arrivals, DevChannel* ch, qm31* alpha,
+                                                                 int m31) {
+  __shared__ TreeSmem sm;
+  const uint32_t L = log_m - fold_step, n = 1u << L;
+  const uint32_t w = min(n, (uint32_t)kTreeThreads), base = blockIdx.x * w, i = base + threadIdx.x;
+  if (threadIdx.x < w) {
+    const qm31 v = CIRCLE ? fold_circle_at(src, itw + (tw_len - n), *d_alpha, i)
+                          : fold_line_at(src.c[0], 1ull << log_m, log_m, fold_step, *d_alpha, itw, tw_len, i);
+    out[i] = v.a;
+    out[n + i] = v.b;
+    out[2 * n + i] = v.c;
+    out[3 * n + i] = v.d;
+    uint32_t h[8];
+    const uint32_t m[16] = {v.a, v.b, v.c, v.d, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    blake2s_init(h);
+    blake2s_compress_lat(h, m, 16, true);
+    dev_finalize(h, m31 != 0);
+    uint4* g = reinterpret_cast<uint4*>(t.out[L] + (size_t)i * 32);
+    g[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    g[1] = make_uint4(h[4], h[5], h[6], h[7]);
+    tree_put(sm.ping, threadIdx.x, h);
+  }
+  __syncthreads();
+  LayerChannel c{ch, alpha, {}};
+  const uint4* root;
+  if (tree_climb<true>(sm, t, L, base, w, 0, gridDim.x > 1 ? arrivals : nullptr, m31 != 0, [&]() { c.begin(); }, &root))
+    c.end(root);
 }
 
 __global__ void __launch_bounds__(kFriTailThreads, 1) fri_tail_kernel(FriTail t, DevChannel* ch, qm31* alphas,
@@ -1804,8 +1834,6 @@ class WideFibProver {
       STWO_CUDA_TRY(cudaEventCreateWithFlags(&ev_tx, cudaEventDisableTiming));
       STWO_CUDA_TRY(
           cudaFuncSetAttribute(fri_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFriTailSmem));
-      STWO_CUDA_TRY(cudaFuncSetAttribute(tree_top_channel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kFriTailSmem));
       STWO_CUDA_TRY(
           cudaFuncSetAttribute(composition_dot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dot_smem(kDotMaxCols)));
       STWO_CUDA_TRY(
@@ -1882,6 +1910,7 @@ class WideFibProver {
     if ((rc = alloc((void**)&d_qdyn, sizeof(QuotientDyn), err, err_len))) return rc;
     h_pinned_bytes = std::max<size_t>(small_q * sizeof(qm31), (16ull << last_log) + (1u << 18));
     if (measure) return 0;
+    STWO_CUDA_TRY(cudaMemsetAsync(d_found + kArrivalsWord, 0, sizeof(uint32_t), s));
     STWO_CUDA_TRY(cudaMallocHost((void**)&h_pinned, h_pinned_bytes));
     h_tx_bytes = 64 + sizeof(FsOut) + (size_t)(N + 8) * sizeof(qm31) + 16;  // + the stream error word
     STWO_CUDA_TRY(cudaMallocHost((void**)&h_tx, h_tx_bytes));
@@ -1939,19 +1968,36 @@ class WideFibProver {
     return 0;
   }
 
-  // One FRI layer tree from its leaf level L: grid-wide node launches down to
-  // 2^kFriTailLog hashes, then one CTA for the top levels (latency-bound, a
-  // few hundred compressions), the root mix and the alpha draw on the device
-  // channel.
+  TreeLevels levels_of(const MerkleTree& t, uint32_t top) const {
+    TreeLevels l;
+    for (uint32_t k = 0; k <= top; k++) l.out[k] = t.layer(k);
+    return l;
+  }
+
+  // One FRI layer tree from its leaf level L: several levels a thread down to
+  // 2^kTreeMaxLog hashes, then one launch for the rest (latency-bound), the
+  // root's mix and the alpha draw on the device channel.
   int fri_tree_top(const MerkleTree& t, uint32_t L, qm31* alpha, char* err, size_t err_len) {
-    const uint32_t top = std::min<uint32_t>(L, kFriTailLog);
+    const uint32_t top = node_levels_wide(L);
     if (L > top) {
       std::vector<uint8_t*> outs(L);
       for (uint32_t k = 0; k < L; k++) outs[k] = t.layer(k);
-      int rc = build_node_layers_impl(t.layer(L), L, top, cfg.m31_channel, outs.data(), s, err, err_len);
+      int rc = build_node_layers_impl(t.layer(L), L, top, cfg.m31_channel, outs.data(), nullptr, s, err, err_len);
       if (rc) return rc;
     }
-    tree_top_channel_kernel<<<1, kFriTailThreads, kFriTailSmem, s>>>(t.base, top, d_chan, alpha, cfg.m31_channel);
+    fri_nodes_kernel<<<tree_blocks(top, kTreeBlockLog), kTreeThreads, 0, s>>>(
+        t.layer(top), top, levels_of(t, top), d_found + kArrivalsWord, d_chan, alpha, cfg.m31_channel);
+    STWO_CHECK_LAUNCH();
+    return 0;
+  }
+
+  // A layer of 2^kFriLayerLog values or fewer from the fold to its alpha.
+  template <bool CIRCLE>
+  int fri_layer(const Src4& src, uint32_t log_m, uint32_t fold_step, const qm31* d_alpha, const FriLayerBuf& l,
+                qm31* alpha, char* err, size_t err_len) {
+    fri_layer_kernel<CIRCLE><<<tree_blocks(l.log_size, 7), kTreeThreads, 0, s>>>(
+        src, log_m, fold_step, d_alpha, d_itw, 1ull << tree_log, l.coords, levels_of(l.tree, l.log_size),
+        d_found + kArrivalsWord, d_chan, alpha, cfg.m31_channel);
     STWO_CHECK_LAUNCH();
     return 0;
   }
@@ -1975,28 +2021,38 @@ class WideFibProver {
     }
     size_t tail0 = fri.size();  // first layer of the fused tail
     while (tail0 > 0 && fri[tail0 - 1].log_size <= kFriTailLog) tail0--;
-    {
+    // Layer `li` (the first from the circle evaluation) with its tree, or the
+    // values below the last tree'd layer.
+    auto is_small = [&](size_t li) { return li < tail0 && fri[li].log_size <= kFriLayerLog; };
+    if (lift <= 4) return set_err(err, err_len, STWO_B200_EARG, "lifting domain too small");
+    const Src4 quot{{d_quot, d_quot + (1ull << lift), d_quot + (2ull << lift), d_quot + (3ull << lift)}};
+    for (size_t li = 0; li <= tail0; li++) {
+      if (li > 0 && li - 1 < tail0 && !is_small(li - 1)) {
+        phase(kFriMerkle);  // leaves were hashed by the fold that produced this layer
+        if ((rc = fri_tree_top(fri[li - 1].tree, fri[li - 1].log_size, d_alphas + li, err, err_len))) return rc;
+      }
+      const FriLayerBuf* from = li > 0 ? &fri[li - 1] : nullptr;
+      if (is_small(li)) {
+        phase(kFriMerkle);
+        rc = from ? fri_layer<false>(Src4{{from->coords, nullptr, nullptr, nullptr}}, from->log_size, from->fold_step,
+                                     d_alphas + li, fri[li], d_alphas + li + 1, err, err_len)
+                  : fri_layer<true>(quot, lift, 1, d_alphas, fri[li], d_alphas + 1, err, err_len);
+        if (rc) return rc;
+        continue;
+      }
       phase(kFriFold);
-      uint32_t* dst = fri.empty() ? d_last : fri[0].coords;
-      uint8_t* leaves = tail0 > 0 ? fri[0].tree.layer(fri[0].log_size) : nullptr;
-      if (lift <= 4) return set_err(err, err_len, STWO_B200_EARG, "lifting domain too small");
-      const Src4 q4{{d_quot, d_quot + (1ull << lift), d_quot + (2ull << lift), d_quot + (3ull << lift)}};
-      fold_circle_first_dev_kernel<<<grid1d(fold_threads(lift - 1), 256), 256, 0, s>>>(
-          q4, lift, d_alphas, d_itw, 1ull << tree_log, dst, leaves, m31 ? 1 : 0);
-      STWO_CHECK_LAUNCH();
-    }
-    for (size_t li = 0; li < tail0; li++) {
-      FriLayerBuf& l = fri[li];
-      phase(kFriMerkle);  // leaves were hashed by the fold that produced this layer
-      if ((rc = fri_tree_top(l.tree, l.log_size, d_alphas + li + 1, err, err_len))) return rc;
-      phase(kFriFold);
-      uint32_t* nxt = (li + 1 < fri.size()) ? fri[li + 1].coords : d_last;
-      uint8_t* leaves = li + 1 < tail0 ? fri[li + 1].tree.layer(fri[li + 1].log_size) : nullptr;
-      uint32_t nlog = l.log_size - l.fold_step;
-      const uint64_t threads = l.fold_step == 1 ? fold_threads(nlog) : 1ull << nlog;
-      fold_line_dev_kernel<<<grid1d(threads, 256), 256, 0, s>>>(l.coords, l.log_size, l.fold_step,
-                                                                       d_alphas + li + 1, d_itw, 1ull << tree_log, nxt,
-                                                                       leaves, m31 ? 1 : 0);
+      uint32_t* dst = li < fri.size() ? fri[li].coords : d_last;
+      uint8_t* leaves = li < tail0 ? fri[li].tree.layer(fri[li].log_size) : nullptr;
+      if (!from) {
+        fold_circle_first_dev_kernel<<<grid1d(fold_threads(lift - 1), 256), 256, 0, s>>>(
+            quot, lift, d_alphas, d_itw, 1ull << tree_log, dst, leaves, m31 ? 1 : 0);
+      } else {
+        const uint32_t nlog = from->log_size - from->fold_step;
+        const uint64_t threads = from->fold_step == 1 ? fold_threads(nlog) : 1ull << nlog;
+        fold_line_dev_kernel<<<grid1d(threads, 256), 256, 0, s>>>(from->coords, from->log_size, from->fold_step,
+                                                                  d_alphas + li, d_itw, 1ull << tree_log, dst, leaves,
+                                                                  m31 ? 1 : 0);
+      }
       STWO_CHECK_LAUNCH();
     }
     if (tail0 < fri.size()) {
@@ -2071,8 +2127,8 @@ class WideFibProver {
                      size_t err_len) {
     std::vector<uint8_t*> layers(t.L + 1);
     for (uint32_t k = 0; k <= t.L; k++) layers[k] = t.layer(k);
-    return stwo_b200_merkle_build_layers(const_cast<const uint32_t* const*>(cols), logs.data(), (uint32_t)logs.size(),
-                                         t.L, cfg.m31_channel, layers.data(), s, err, err_len);
+    return build_layers_impl(const_cast<const uint32_t* const*>(cols), logs.data(), (uint32_t)logs.size(), t.L,
+                             cfg.m31_channel, layers.data(), d_found + kArrivalsWord, s, err, err_len);
   }
 
   int prove(const uint32_t* d_a, const uint32_t* d_b, ProofOut& out, char* err, size_t err_len,
@@ -2767,6 +2823,7 @@ struct SeededFriProver {
   uint8_t* d_gather_out = nullptr;
   size_t gather_cap = 0;     // entries (words or hashes)
   uint8_t* h_stage = nullptr;  // pinned: addresses (8 B / entry), then gathered bytes (32 B / entry)
+  uint32_t* d_arrivals = nullptr;  // a word for each tree: they are built side by side
   // the commit sequence, captured once per input column set
   cudaGraphExec_t exec = nullptr;
   const void* key[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -2815,6 +2872,8 @@ struct SeededFriProver {
       if ((rc = alloc((void**)&trees[k].base, MerkleTree::bytes_for(n - k), err, err_len))) return rc;
     }
     if ((rc = alloc((void**)&d_alphas, n * sizeof(qm31), err, err_len))) return rc;
+    if ((rc = alloc((void**)&d_arrivals, n * sizeof(uint32_t), err, err_len))) return rc;
+    STWO_CUDA_TRY(cudaMemsetAsync(d_arrivals, 0, n * sizeof(uint32_t), s));
     STWO_CUDA_TRY(cudaMallocHost((void**)&h_alphas, n * sizeof(qm31)));
     return 0;
   }
@@ -2841,7 +2900,7 @@ struct SeededFriProver {
       STWO_CUDA_TRY(cudaEventRecord(ev_fork[k], s));
       STWO_CUDA_TRY(cudaStreamWaitEvent(x, ev_fork[k], 0));
       auto lk = layer_ptrs(trees[k]);
-      return build_node_layers_impl(trees[k].layer(L), L, 0, m31, lk.data(), x, err, err_len);
+      return build_node_layers_impl(trees[k].layer(L), L, 0, m31, lk.data(), d_arrivals + k, x, err, err_len);
     };
     {
       // the circle layer's whole tree reads only the input columns: it runs
@@ -2851,7 +2910,7 @@ struct SeededFriProver {
       STWO_CUDA_TRY(cudaStreamWaitEvent(x, ev_fork[0], 0));
       if ((rc = build_leaves_impl(d_coords, lg, 4, n, m31, trees[0].layer(n), nullptr, x, err, err_len))) return rc;
       auto l0 = layer_ptrs(trees[0]);
-      if ((rc = build_node_layers_impl(trees[0].layer(n), n, 0, m31, l0.data(), x, err, err_len))) return rc;
+      if ((rc = build_node_layers_impl(trees[0].layer(n), n, 0, m31, l0.data(), d_arrivals, x, err, err_len))) return rc;
     }
     const Src4 src{{d_coords[0], d_coords[1], d_coords[2], d_coords[3]}};
     fold_circle_first_dev_kernel<<<grid1d(fold_threads(n - 1), 256), 256, 0, s>>>(
