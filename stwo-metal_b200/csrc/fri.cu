@@ -95,6 +95,39 @@ __global__ void __launch_bounds__(256) fold_line2_kernel(Cols4 in, uint32_t log_
   }
 }
 
+// fold_line with fold_step 2 or 3, one output per thread: its 2^STEP inputs are
+// whole 16-byte loads of each coordinate and stay in registers (the general
+// kernel indexes them at run time, in local memory, and loads word by word).
+// Same arithmetic per output.  Inputs 16-byte aligned.
+template <int STEP>
+__global__ void __launch_bounds__(256) fold_line_steps_kernel(Cols4 in, uint32_t log_m, FoldAlphas alphas,
+                                                              const uint32_t* itw, uint64_t tw_len, Cols4W out) {
+  const uint64_t n_out = 1ull << (log_m - STEP);
+  for (uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; o < n_out; o += (uint64_t)gridDim.x * blockDim.x) {
+    qm31 v[1 << STEP];
+#pragma unroll
+    for (int q = 0; q < (1 << STEP) / 4; q++) {
+      uint4 w[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) w[c] = __ldg(reinterpret_cast<const uint4*>(in.c[c]) + (o << (STEP - 2)) + q);
+      v[4 * q] = {w[0].x, w[1].x, w[2].x, w[3].x};
+      v[4 * q + 1] = {w[0].y, w[1].y, w[2].y, w[3].y};
+      v[4 * q + 2] = {w[0].z, w[1].z, w[2].z, w[3].z};
+      v[4 * q + 3] = {w[0].w, w[1].w, w[2].w, w[3].w};
+    }
+#pragma unroll
+    for (int s = 0; s < STEP; s++) {
+      const uint32_t* lt = itw + (tw_len - (1ull << (log_m - s))) + (o << (STEP - 1 - s));
+#pragma unroll
+      for (int j = 0; j < (1 << (STEP - 1 - s)); j++) {
+        const qm31 fx = v[2 * j], fnx = v[2 * j + 1];
+        v[j] = qm31_add(qm31_add(fx, fnx), qm31_mul(alphas.a[s], qm31_mul_m31(qm31_sub(fx, fnx), __ldg(lt + j))));
+      }
+    }
+    store_q(out, o, v[0]);
+  }
+}
+
 // Circle-layer inverse twiddle of pair i, derived from line layer 1 of the
 // source domain: [y, -y, -x, x] (simd/fft/mod.rs:61-97).
 __device__ __forceinline__ uint32_t circle_itw(const uint32_t* lt0, uint64_t i) {
@@ -252,6 +285,12 @@ extern "C" int stwo_b200_fold_line(const uint32_t* const* d_in4, uint32_t log_si
       aligned4(reinterpret_cast<const void* const*>(out.c), 8))
     fold_line2_kernel<<<grid_for(n_out / 2, 256), 256, 0, as_stream(stream)>>>(in, log_size, al.a[0], d_itwiddles,
                                                                               1ull << tree_log_size, out);
+  else if (fold_step == 2 && aligned4(reinterpret_cast<const void* const*>(in.c), 16))
+    fold_line_steps_kernel<2><<<grid_for(n_out, 256), 256, 0, as_stream(stream)>>>(in, log_size, al, d_itwiddles,
+                                                                                   1ull << tree_log_size, out);
+  else if (fold_step == 3 && aligned4(reinterpret_cast<const void* const*>(in.c), 16))
+    fold_line_steps_kernel<3><<<grid_for(n_out, 256), 256, 0, as_stream(stream)>>>(in, log_size, al, d_itwiddles,
+                                                                                   1ull << tree_log_size, out);
   else
     fold_line_kernel<<<grid_for(n_out, 256), 256, 0, as_stream(stream)>>>(in, log_size, fold_step, al, d_itwiddles,
                                                                           1ull << tree_log_size, out);
