@@ -1,5 +1,5 @@
-"""Folds of two and three layers at word-aligned columns (the general kernel) and
-at 16-byte aligned ones (whole loads), against the oracle."""
+"""Folds of two and three layers and lifted sums at word-aligned columns (the
+general kernels) and at 16-byte aligned ones (whole loads), against the oracle."""
 import numpy as np
 import pytest
 
@@ -36,4 +36,14 @@ def test_fold_line_steps(step, log, at):
     alpha = np.random.default_rng(log).integers(0, P, 4, dtype=np.uint32)
     got = be.fold_line(col, alpha, tree, step).to_host()
     for a, b in zip(got, oracle.fold_line(w, itw, alpha, step)):
+        assert (a == b).all()
+
+
+@pytest.mark.parametrize("at", [0, 1, 2, 4])
+@pytest.mark.parametrize("logs", [[1], [2], [5], [1, 2], [1, 3], [2, 3, 4, 5], [1, 9], [3, 4, 11, 17], [16, 17]])
+def test_lifted_sums(logs, at):
+    be = B200Backend()
+    cols = [column(g, 50 + g, at) for g in logs]
+    ref = oracle.lift_and_accumulate([w for _, w in cols])
+    for a, b in zip(be.lift_and_accumulate([c for c, _ in cols]).to_host(), ref):
         assert (a == b).all()
