@@ -4,11 +4,15 @@
 // every SIGMA index is a compile-time constant.  Rotations by 16 and 8 are byte
 // permutes, by 12 and 7 funnel shifts.  Two forms of the same function:
 //  - blake2s_compress (throughput): XORs and rotations keep the integer ALU
-//    pipe busy, so the additions go to the multiply-add pipe: x + y is written
-//    x * kB2sOne + y with kB2sOne a constant-bank 1 that the compiler cannot
-//    fold.  About 20% more compressions per second on a full GPU.
+//    pipe busy, so the message word is added on the multiply-add pipe, as
+//    x * 1 + a with a 1 that the compiler cannot fold; b and c are plain
+//    two-input additions.  With all four additions of a G there (as before),
+//    they bound it: FRI proof of 2^24, 6.7e7 compressions, 3171 -> 3038 us,
+//    100 x 2^20 proof 3852 -> 3810, 512-column commit 13176 -> 13067.  With the
+//    second or both additions to a there: 3075 us.
 //  - blake2s_compress_lat (latency): a + b + m as one three-input add, the
-//    shortest dependency chain, for the one-CTA tree tops and channel steps.
+//    shortest dependency chain, for the one-CTA tree tops and channel steps
+//    (the other form there: 2^10-row proof 354 -> 362 us).
 // This is the hash of crate blake2 0.10.6 as called by stwo
 // (crates/stwo/src/core/vcs/blake2_hash.rs:84-94).
 #pragma once
@@ -27,17 +31,21 @@ __device__ __forceinline__ uint32_t rotr7(uint32_t x) { return __funnelshift_r(x
 
 // 1, but not a compile-time constant (see the header comment).
 __device__ __constant__ uint32_t kB2sOne = 1;
-__device__ __forceinline__ uint32_t madd(uint32_t x, uint32_t y) { return x * kB2sOne + y; }
+__device__ __forceinline__ uint32_t madd(uint32_t x, uint32_t y) {
+  uint32_t r;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(x), "r"(kB2sOne), "r"(y));
+  return r;
+}
 
 #define STWO_B2S_G(a, b, c, d, x, y)      \
   do {                                    \
-    v[a] = madd(v[b], madd((x), v[a]));   \
+    v[a] = v[b] + madd((x), v[a]);        \
     v[d] = rotr16(v[d] ^ v[a]);           \
-    v[c] = madd(v[d], v[c]);              \
+    v[c] = v[d] + v[c];                   \
     v[b] = rotr12(v[b] ^ v[c]);           \
-    v[a] = madd(v[b], madd((y), v[a]));   \
+    v[a] = v[b] + madd((y), v[a]);        \
     v[d] = rotr8(v[d] ^ v[a]);            \
-    v[c] = madd(v[d], v[c]);              \
+    v[c] = v[d] + v[c];                   \
     v[b] = rotr7(v[b] ^ v[c]);            \
   } while (0)
 
