@@ -358,20 +358,20 @@ __global__ void bit_reverse_cols_kernel(FftCols t, uint32_t log_n) {
 // The same for columns of at least 2^10 words, through shared memory.  With i =
 // (a, m, b), 5 high bits a and 5 low bits b, word (a, m, b) goes to (rev b, rev
 // m, rev a): the 32 x 32 words of one middle part m, 32 rows of 128 contiguous
-// bytes, become those of rev m.  A block moves tile m, and in place tile rev m
-// with it (the block of the smaller of the two), so every sector is read and
+// bytes, become those of rev m.  A block moves tile m and tile rev m with it (the
+// block of the smaller of the two): in place it has to, and out of place it
+// doubles the bytes that a thread has in flight.  Every sector is read and
 // written whole, once; word by word each 4-byte access moves a 32-byte sector.
 // Bound by HBM: four columns of 2^20 in place 81 -> 7 us, 37 columns of 2^19 out
-// of place 131 -> 34 us, against the word swaps.
+// of place 131 -> 34 us, against the word swaps, and 27 us by two tiles.
 __global__ void __launch_bounds__(256) bit_reverse_tiles_kernel(FftCols t, uint32_t log_n) {
   __shared__ uint32_t tile[2][32][33];
   const uint32_t* src = t.src[blockIdx.y];
   uint32_t* dst = t.dst[blockIdx.y];
-  const bool in_place = src == dst;
   const uint32_t mid = log_n - 10, m = blockIdx.x, rm = mid ? __brev(m) >> (32 - mid) : 0;
-  if (in_place && m > rm) return;
+  if (m > rm) return;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool both = in_place && m != rm;
+  const bool both = m != rm;
 #pragma unroll
   for (uint32_t u = 0; u < 4; u++) {
     const uint32_t a = warp + 8 * u;
