@@ -859,7 +859,7 @@ def run_prove_b200(args, world, rank, local):
     kind, amount = alg[dominant]
     if kind == "int32":
         achieved = amount / (ph[dominant] * 1e-3) / 1e9
-        roof = {"bound": "int32", "kernel": dominant + " (lifted_leaves_kernel + node_layers_kernel)",
+        roof = {"bound": "int32", "kernel": dominant + " (lifted_leaves_kernel + node_levels_kernel)",
                 "achieved": achieved, "peak": probe_rate / 1e9, "unit": "G Blake2s compressions/s",
                 "frac": achieved * 1e9 / probe_rate,
                 "peak_kind": "measured in this run (register-only Blake2s chain, all SMs)", "traffic": None,
@@ -1087,7 +1087,7 @@ def run_fri_b200(args, world, rank, local):
     # layer k and are a small share.
     compressions = sum((1 << (k + 1)) - 1 for k in range(1, FRI_LOG + 1))
     achieved = compressions / (ms * 1e-3) / 1e9
-    roof = {"bound": "int32", "kernel": "Blake2s trees of every layer (lifted_leaves_kernel + node_layers_kernel)",
+    roof = {"bound": "int32", "kernel": "Blake2s trees of every layer (lifted_leaves_kernel + node_levels_kernel)",
             "achieved": achieved, "peak": probe_rate / 1e9, "unit": "G Blake2s compressions/s",
             "frac": achieved * 1e9 / probe_rate,
             "peak_kind": "measured in this run (register-only Blake2s chain, all SMs)", "traffic": None,

@@ -338,6 +338,9 @@ int build_leaves_impl(const uint32_t* const* d_cols, const uint32_t* log_sizes, 
   return STWO_B200_OK;
 }
 
+// From 2^18 hashes on a thread hashes three levels at a time (2^15 threads then,
+// two warps a scheduler): with 2^18 left to one launch a proof of 173 x 2^17
+// took 1334 us instead of 1312, of 100 x 2^20 3906 instead of 3871.
 constexpr uint32_t kSubtree3MinLog = 18;
 uint32_t node_levels_wide(uint32_t L) {
   while (L >= kSubtree3MinLog) L -= 3;
