@@ -67,8 +67,6 @@ int stwo_b200_memcpy_d2d(void* d_dst, const void* d_src, size_t bytes, void* str
 int stwo_b200_memset(void* d_dst, int value, size_t bytes, void* stream, char* err, size_t err_len);
 int stwo_b200_stream_create(void** stream_out, char* err, size_t err_len);
 int stwo_b200_stream_destroy(void* stream, char* err, size_t err_len);
-/* Waits for the stream.  STWO_B200_ETIMEOUT (once) when a bounded device wait
- * of an operation enqueued before has given up; its outputs are incomplete. */
 int stwo_b200_stream_sync(void* stream, char* err, size_t err_len);
 /* Pinned host memory for the e2e copies. */
 int stwo_b200_host_alloc(size_t bytes, void** h_out, char* err, size_t err_len);
@@ -285,6 +283,15 @@ typedef struct stwo_b200_sample_batch {
 int stwo_b200_accumulate_numerators(const uint32_t* const* d_cols, uint32_t n_cols, uint32_t log_size,
                                     const stwo_b200_sample_batch* batches, uint32_t n_batches, uint32_t* const* d_out,
                                     uint32_t* first_linear_term_out, void* stream, char* err, size_t err_len);
+/* The same with a bound for the device waits of its tensor-core form: a thread
+ * polls at most `polls` times and takes its remaining rows on the integer pipes
+ * when that runs out.  The call above uses STWO_B200_STREAM_SPIN_DEFAULT; 0
+ * gives up at the first wait, with the same results.  No reference counterpart:
+ * this exercises that path. */
+int stwo_b200_accumulate_numerators_polls(const uint32_t* const* d_cols, uint32_t n_cols, uint32_t log_size,
+                                          const stwo_b200_sample_batch* batches, uint32_t n_batches,
+                                          uint32_t* const* d_out, uint32_t* first_linear_term_out, uint32_t polls,
+                                          void* stream, char* err, size_t err_len);
 
 /* AccumulatedNumerators (prover/pcs/quotient_ops.rs:48-74) of one sample point:
  * the partial numerator's 4 device coordinate columns of 2^log_size words and
@@ -335,6 +342,14 @@ int stwo_b200_lift_and_accumulate(const uint32_t* const* d_cols4, const uint32_t
 int stwo_b200_batch_eval_at_point(const uint32_t* const* d_coeffs, uint32_t n_polys, uint32_t log_size,
                                   const uint32_t* point, uint32_t* values_out, void* stream, char* err,
                                   size_t err_len);
+/* The same with a bound for the device waits of its tensor-core form: when one
+ * runs out after `polls` polls, this call returns STWO_B200_ETIMEOUT and leaves
+ * values_out as it was.  The call above uses STWO_B200_STREAM_SPIN_DEFAULT; 0
+ * gives up at the first wait.  No reference counterpart: this exercises the
+ * failure path. */
+int stwo_b200_batch_eval_at_point_polls(const uint32_t* const* d_coeffs, uint32_t n_polys, uint32_t log_size,
+                                        const uint32_t* point, uint32_t* values_out, uint32_t polls, void* stream,
+                                        char* err, size_t err_len);
 /* PolyOps::eval_at_point (ops.rs:44-48) of one polynomial. */
 int stwo_b200_eval_at_point(const uint32_t* d_coeffs, uint32_t log_size, const uint32_t* point, uint32_t* value_out,
                             void* stream, char* err, size_t err_len);

@@ -48,14 +48,6 @@ inline cudaError_t ensure_smem_limit(Kernel* kernel, int bytes, std::atomic<uint
 // Number of kernels this library has launched (read by stwo_b200_launch_count).
 extern std::atomic<uint64_t> g_kernel_launches;
 
-// One word of pinned host memory that a kernel sets when a bounded device wait
-// of its own gives up (no such wait runs out unless the device is broken); the
-// synchronising calls return STWO_B200_ETIMEOUT once for it.  Made by
-// stwo_b200_init and kept until the process ends; nullptr before.
-uint32_t* fault_word();
-// Whether it was set since the last call.
-bool take_fault();
-
 // Host/device index helpers.
 __host__ __device__ __forceinline__ uint32_t bitrev32(uint32_t x, uint32_t bits) {
 #ifdef __CUDA_ARCH__

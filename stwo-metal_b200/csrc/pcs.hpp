@@ -19,14 +19,16 @@ uint32_t poly_eval_lo_bits(uint32_t lg);
 // Values at one point of n_polys (<= 1024) polynomials of 2^lg natural-order
 // coefficients each, from the weight tables of launch_eval_weights (w_lo:
 // 2^h entries, w_hi: 2^(lg - h), h = poly_eval_lo_bits(lg)):
-// d_out[p] = sum_j coeff_p[j] w_j.  *fault (when given) is set if a bounded
-// device wait gave up.
+// d_out[p] = sum_j coeff_p[j] w_j.  A device wait polls at most `spin` times;
+// *fault (device memory, cleared before by the caller) is set if one gave up,
+// and the values are incomplete then.
 int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg, const qm31* d_w_lo,
-                     const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, cudaStream_t s, char* err,
-                     size_t err_len);
-// Weight tables of the point z for polynomials of 2^lg coefficients.
-int launch_eval_weights(const spoint& z, uint32_t lg, qm31* d_w_lo, qm31* d_w_hi, cudaStream_t s, char* err,
-                        size_t err_len);
+                     const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, uint32_t spin, cudaStream_t s,
+                     char* err, size_t err_len);
+// Weight tables of the point z for polynomials of 2^lg coefficients; clears
+// *fault.
+int launch_eval_weights(const spoint& z, uint32_t lg, qm31* d_w_lo, qm31* d_w_hi, uint32_t* fault, cudaStream_t s,
+                        char* err, size_t err_len);
 // One proof-of-work batch: nonces (hi << 32) | (low_base + t), t < count
 // (a multiple of 256), prefixed digest `pre`; the smallest hit is
 // atomicMin'ed into *d_found.

@@ -22,6 +22,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "channel.hpp"
@@ -50,55 +52,63 @@ struct NumeratorTerms {
   qm31 c[kNumTerms];
 };
 
+// Rows i .. i + R - 1 (R = 4: columns 16-byte aligned) on the integer pipes.
+template <int R>
+__device__ __forceinline__ void numerators_rows(const NumeratorTerms& t, uint32_t n_terms, const qm31& b_sum,
+                                                int accumulate, const Col4& out, uint64_t i) {
+  acc4 s[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) s[r] = {0, 0, 0, 0};
+  for (uint32_t k = 0; k < n_terms; k++) {
+    const qm31 c = t.c[k];
+    if (R == 4) {
+      const uint4 v = ldg4(t.col[k] + i);
+#pragma unroll
+      for (int r = 0; r < R; r++) acc4_mad(s[r], c, u4get(v, r));
+    } else {
+      acc4_mad(s[0], c, __ldg(t.col[k] + i));
+    }
+    if ((k & 3) == 3) {
+#pragma unroll
+      for (int r = 0; r < R; r++) acc4_fold(s[r]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    qm31 v = acc4_reduce(s[r]);
+    if (accumulate)
+      v = qm31_add(qm31{out.c[0][i + r], out.c[1][i + r], out.c[2][i + r], out.c[3][i + r]}, v);
+    else
+      v = qm31_sub(v, b_sum);
+    out.c[0][i + r] = v.a;
+    out.c[1][i + r] = v.b;
+    out.c[2][i + r] = v.c;
+    out.c[3][i + r] = v.d;
+  }
+}
+
 template <bool VEC>
 __global__ void __launch_bounds__(256) numerators_kernel(NumeratorTerms t, uint32_t n_terms, qm31 b_sum, uint64_t n,
                                                          int accumulate, Col4 out) {
   constexpr int R = VEC ? 4 : 1;
   const uint64_t n_units = n / R;
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n_units;
-       u += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = u * R;
-    acc4 s[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) s[r] = {0, 0, 0, 0};
-    for (uint32_t k = 0; k < n_terms; k++) {
-      const qm31 c = t.c[k];
-      if (VEC) {
-        const uint4 v = ldg4(t.col[k] + i);
-#pragma unroll
-        for (int r = 0; r < R; r++) acc4_mad(s[r], c, u4get(v, r));
-      } else {
-        acc4_mad(s[0], c, __ldg(t.col[k] + i));
-      }
-      if ((k & 3) == 3) {
-#pragma unroll
-        for (int r = 0; r < R; r++) acc4_fold(s[r]);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      qm31 v = acc4_reduce(s[r]);
-      if (accumulate)
-        v = qm31_add(qm31{out.c[0][i + r], out.c[1][i + r], out.c[2][i + r], out.c[3][i + r]}, v);
-      else
-        v = qm31_sub(v, b_sum);
-      out.c[0][i + r] = v.a;
-      out.c[1][i + r] = v.b;
-      out.c[2][i + r] = v.c;
-      out.c[3][i + r] = v.d;
-    }
-  }
+       u += (uint64_t)gridDim.x * blockDim.x)
+    numerators_rows<R>(t, n_terms, b_sum, accumulate, out, u * R);
 }
 
 // The same sums on the tensor cores (rowdot.cuh): whole 512-row tiles, columns
-// and outputs 16-byte aligned.
+// and outputs 16-byte aligned.  The call returns before the kernel has run, so
+// a wait that gives up has nobody to report to: its thread takes the rows it
+// is left with on the integer pipes.
 __global__ void __launch_bounds__(kDotThreads, kDotBlocks) numerators_dot_kernel(NumeratorTerms t, uint32_t n_terms,
                                                                        qm31 b_sum, uint64_t n, int accumulate,
-                                                                       Col4 out, uint32_t* err) {
+                                                                       Col4 out, uint32_t spin) {
   extern __shared__ __align__(1024) uint8_t sm8[];
   const NumeratorTerms* tp = &t;
-  row_dot(
-      sm8, n_terms, (uint32_t)(n >> kDotTileBits), kStreamSpin, err, [=](uint32_t k) { return tp->col[k]; },
+  const uint32_t n_tiles = (uint32_t)(n >> kDotTileBits);
+  uint32_t left = row_dot(
+      sm8, n_terms, n_tiles, spin, nullptr, [=](uint32_t k) { return tp->col[k]; },
       [=](uint32_t k) { return tp->c[k]; }, []() {}, [](int, uint32_t x) { return x; },
       [&](uint32_t tile, const qm31(&s)[4]) {
         const uint64_t i = ((uint64_t)tile << kDotTileBits) + 4 * threadIdx.x;
@@ -119,6 +129,9 @@ __global__ void __launch_bounds__(kDotThreads, kDotBlocks) numerators_dot_kernel
         *reinterpret_cast<uint4*>(out.c[2] + i) = make_uint4(v[0].c, v[1].c, v[2].c, v[3].c);
         *reinterpret_cast<uint4*>(out.c[3] + i) = make_uint4(v[0].d, v[1].d, v[2].d, v[3].d);
       });
+#pragma unroll 1
+  for (; left < n_tiles; left += gridDim.x)
+    numerators_rows<4>(t, n_terms, b_sum, accumulate, out, ((uint64_t)left << kDotTileBits) + 4 * threadIdx.x);
 }
 
 // ------------------------------------------------- lift_and_accumulate -----
@@ -320,6 +333,14 @@ extern "C" int stwo_b200_accumulate_numerators(const uint32_t* const* d_cols, ui
                                                const stwo_b200_sample_batch* batches, uint32_t n_batches,
                                                uint32_t* const* d_out, uint32_t* first_linear_term_out,
                                                void* stream, char* err, size_t err_len) {
+  return stwo_b200_accumulate_numerators_polls(d_cols, n_cols, log_size, batches, n_batches, d_out,
+                                               first_linear_term_out, kStreamSpin, stream, err, err_len);
+}
+
+extern "C" int stwo_b200_accumulate_numerators_polls(const uint32_t* const* d_cols, uint32_t n_cols, uint32_t log_size,
+                                                     const stwo_b200_sample_batch* batches, uint32_t n_batches,
+                                                     uint32_t* const* d_out, uint32_t* first_linear_term_out,
+                                                     uint32_t polls, void* stream, char* err, size_t err_len) {
   STWO_ARG_CHECK(n_batches == 0 || (batches && d_out && first_linear_term_out), "null argument");
   STWO_ARG_CHECK(log_size <= 30, "log size %u too large", log_size);
   cudaStream_t s = as_stream(stream);
@@ -371,7 +392,7 @@ extern "C" int stwo_b200_accumulate_numerators(const uint32_t* const* d_cols, ui
         static std::atomic<uint32_t> attr{0};
         STWO_CUDA_TRY(ensure_smem_limit(numerators_dot_kernel, (int)dot_smem(kNumTerms), attr));
         numerators_dot_kernel<<<dot_grid(dot_smem(nt), 0, (uint32_t)(n >> kDotTileBits)),
-                                kDotThreads, dot_smem(nt), s>>>(t, nt, b_sum, n, acc, out, fault_word());
+                                kDotThreads, dot_smem(nt), s>>>(t, nt, b_sum, n, acc, out, polls);
       } else if (aligned)
         numerators_kernel<true><<<grid_rows(n / 4, 256), 256, 0, s>>>(t, nt, b_sum, n, acc, out);
       else
@@ -495,6 +516,13 @@ extern "C" int stwo_b200_generate_secure_powers(const uint32_t* felt, uint32_t n
 extern "C" int stwo_b200_batch_eval_at_point(const uint32_t* const* d_coeffs, uint32_t n_polys, uint32_t log_size,
                                              const uint32_t* point, uint32_t* values_out, void* stream, char* err,
                                              size_t err_len) {
+  return stwo_b200_batch_eval_at_point_polls(d_coeffs, n_polys, log_size, point, values_out, kStreamSpin, stream, err,
+                                             err_len);
+}
+
+extern "C" int stwo_b200_batch_eval_at_point_polls(const uint32_t* const* d_coeffs, uint32_t n_polys,
+                                                   uint32_t log_size, const uint32_t* point, uint32_t* values_out,
+                                                   uint32_t polls, void* stream, char* err, size_t err_len) {
   STWO_ARG_CHECK(point && (n_polys == 0 || (d_coeffs && values_out)), "null argument");
   STWO_ARG_CHECK(log_size <= 30, "log size %u too large", log_size);
   STWO_ARG_CHECK(canonical4(point) && canonical4(point + 4), "point not canonical");
@@ -513,26 +541,33 @@ extern "C" int stwo_b200_batch_eval_at_point(const uint32_t* const* d_coeffs, ui
   const uint32_t lg = log_size, h = poly_eval_lo_bits(lg);
   const uint32_t n_chunk_polys = std::min<uint32_t>(n_polys, kMaxPolys);
   const size_t n_w = (1ull << h) + (1ull << (lg - h));
-  const size_t words = n_w + (size_t)n_chunk_polys * poly_eval_chunks(lg) + n_polys;
+  const size_t words = n_w + (size_t)n_chunk_polys * poly_eval_chunks(lg) + n_polys + 1;
+  // the values and, behind them, whether a device wait gave up: one copy
+  const size_t out_bytes = (size_t)n_polys * sizeof(qm31);
+  std::unique_ptr<uint32_t[]> host(new (std::nothrow) uint32_t[4 * (size_t)n_polys + 1]);
+  if (!host) return set_err(err, err_len, STWO_B200_ENOMEM, "no host memory for the values");
   qm31* scratch = nullptr;
   STWO_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&scratch), words * sizeof(qm31), s));
   qm31* w_lo = scratch;
   qm31* w_hi = scratch + (1ull << h);
   qm31* partial = scratch + n_w;
   qm31* vals = partial + (size_t)n_chunk_polys * poly_eval_chunks(lg);
-  int rc = launch_eval_weights(z, lg, w_lo, w_hi, s, err, err_len);
+  uint32_t* fault = reinterpret_cast<uint32_t*>(vals + n_polys);
+  int rc = launch_eval_weights(z, lg, w_lo, w_hi, fault, s, err, err_len);
   for (uint32_t p0 = 0; rc == 0 && p0 < n_polys; p0 += kMaxPolys) {
     const uint32_t np = std::min<uint32_t>(kMaxPolys, n_polys - p0);
-    rc = launch_poly_eval(d_coeffs + p0, np, lg, w_lo, w_hi, partial, vals + p0, fault_word(), s, err, err_len);
+    rc = launch_poly_eval(d_coeffs + p0, np, lg, w_lo, w_hi, partial, vals + p0, fault, polls, s, err, err_len);
   }
   if (rc == 0) {
-    const cudaError_t e = cudaMemcpyAsync(values_out, vals, (size_t)n_polys * sizeof(qm31), cudaMemcpyDeviceToHost, s);
+    const cudaError_t e = cudaMemcpyAsync(host.get(), vals, out_bytes + sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) rc = set_err(err, err_len, STWO_B200_ECUDA, "copy of the values: %s", cudaGetErrorString(e));
   }
   cudaFreeAsync(scratch, s);
   if (rc) return rc;
   STWO_CUDA_TRY(cudaStreamSynchronize(s));
-  if (take_fault()) return set_err(err, err_len, STWO_B200_ETIMEOUT, "a tensor-core product did not complete in time");
+  if (host[4 * (size_t)n_polys])
+    return set_err(err, err_len, STWO_B200_ETIMEOUT, "a tensor-core product did not complete in time");
+  std::memcpy(values_out, host.get(), out_bytes);
   return ok(err, err_len);
 }
 

@@ -294,7 +294,8 @@ constexpr size_t kEvalDotSmem = ((1u << kEvalLoBits) / 32) * kDotStage + 2 * kEv
 __global__ void __launch_bounds__(256, 1) poly_eval_dot_kernel(PolyTable t, uint32_t n_polys, uint32_t n_buckets,
                                                                const qm31* __restrict__ w_lo,
                                                                const qm31* __restrict__ w_hi,
-                                                               qm31* __restrict__ partial, uint32_t* err) {
+                                                               qm31* __restrict__ partial, uint32_t* err,
+                                                               uint32_t spin) {
   extern __shared__ __align__(1024) uint8_t sm8[];
   uint8_t* opB = sm8;
   uint8_t* opA = sm8 + ((1u << kEvalLoBits) / 32) * kDotStage;
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(256, 1) poly_eval_dot_kernel(PolyTable t, uint
       }
       umma_commit(&sy->bar[g & 1]);
     }
-    ok = ok && mbar_wait(&sy->bar[g & 1], (g >> 1) & 1);
+    ok = ok && mbar_wait(&sy->bar[g & 1], (g >> 1) & 1, spin);
     fill(g + 2);
     if (in_bucket + 1 == kEvalPerBucket && tid < 128) {
       umma_fence_after();
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(256, 1) poly_eval_dot_kernel(PolyTable t, uint
       umma_commit(&sy->drain);
       (void)mbar_wait(&sy->drain, 0);
     }
-    if (err) *err = 1;
+    *err = 1;
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   umma_fence_before();
@@ -397,8 +398,8 @@ uint32_t poly_eval_lo_bits(uint32_t lg) { return lg >= 13 && lg <= 24 ? kEvalLoB
 // rows would be empty.
 constexpr uint32_t kEvalDotPolys = 32;
 int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg, const qm31* d_w_lo,
-                     const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, cudaStream_t s, char* err,
-                     size_t err_len) {
+                     const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, uint32_t spin, cudaStream_t s,
+                     char* err, size_t err_len) {
   STWO_ARG_CHECK(n_polys >= 1 && n_polys <= (uint32_t)kMaxPolys && lg <= 30, "poly eval: bad shape");
   PolyTable pt;
   bool aligned = true;  // for 16-byte loads; other pointers take the chunked form
@@ -417,7 +418,7 @@ int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg
       const uint32_t groups = (n_polys + 127) / 128, buckets = 1u << (lg - h);
       const uint32_t blocks = std::min(buckets, std::max(1u, 148u / groups));
       poly_eval_dot_kernel<<<dim3(blocks, groups), 256, kEvalDotSmem, s>>>(pt, n_polys, buckets, d_w_lo, d_w_hi,
-                                                                           d_partial, fault);
+                                                                           d_partial, fault, spin);
       STWO_CHECK_LAUNCH();
       oods_reduce_kernel<<<n_polys, 256, 0, s>>>(d_partial, blocks, d_out);
       STWO_CHECK_LAUNCH();
@@ -1078,9 +1079,10 @@ __global__ void fs_oods_kernel(DevChannel* ch, const uint8_t* root, uint32_t lg,
 // The weight tables of oods_eval_kernel for an explicit point z
 // (PolyOps::batch_eval_at_point): f = [y, x, pi(x), ...] of z, then as above.
 __global__ void eval_weights_kernel(spoint z, uint32_t lg, uint32_t h, qm31* __restrict__ w_lo,
-                                    qm31* __restrict__ w_hi) {
+                                    qm31* __restrict__ w_hi, uint32_t* __restrict__ fault) {
   __shared__ qm31 f[32];
   if (threadIdx.x == 0) {
+    *fault = 0;
     f[0] = z.y;
     qm31 xx = z.x;
     for (uint32_t b = 1; b < lg; b++) {
@@ -1092,9 +1094,9 @@ __global__ void eval_weights_kernel(spoint z, uint32_t lg, uint32_t h, qm31* __r
   build_eval_weights(f, lg, h, w_lo, w_hi);
 }
 
-int launch_eval_weights(const spoint& z, uint32_t lg, qm31* d_w_lo, qm31* d_w_hi, cudaStream_t s, char* err,
-                        size_t err_len) {
-  eval_weights_kernel<<<1, 1024, 0, s>>>(z, lg, poly_eval_lo_bits(lg), d_w_lo, d_w_hi);
+int launch_eval_weights(const spoint& z, uint32_t lg, qm31* d_w_lo, qm31* d_w_hi, uint32_t* fault, cudaStream_t s,
+                        char* err, size_t err_len) {
+  eval_weights_kernel<<<1, 1024, 0, s>>>(z, lg, poly_eval_lo_bits(lg), d_w_lo, d_w_hi, fault);
   STWO_CHECK_LAUNCH();
   return STWO_B200_OK;
 }
@@ -2306,7 +2308,7 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     for (int k = 0; k < 8; k++) polys.push_back(split[k]);
     d_vals = d_small + n_w;
     if ((rc = launch_poly_eval(polys.data(), np, lg, d_small, d_small + (1u << h), d_oods_partial, d_vals,
-                               d_found + kStreamErrWord, s, err, err_len)))
+                               d_found + kStreamErrWord, kStreamSpin, s, err, err_len)))
       return rc;
   }
 

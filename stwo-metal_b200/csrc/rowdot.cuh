@@ -56,11 +56,13 @@ __host__ __device__ constexpr size_t dot_smem(uint32_t n_cols) {
 //                    past the last column (whose weights are zero),
 //   rows(tile, s)    the tile's sums of this thread's 4 rows.
 // `sm8`: dot_smem(n_cols) bytes, 1024-byte aligned.  Every wait polls at most
-// `spin` times; a thread whose wait ran out sets *err, waits no more and
-// writes no rows.
+// `spin` times; a thread whose wait ran out sets *err (if given), waits no more
+// and has no more rows.  Returns the first of the block's tiles whose sums this
+// thread did not get: n_tiles or above when it got them all.
 template <typename ColFn, typename WeightFn, typename BeginFn, typename WordFn, typename RowsFn>
-__device__ __forceinline__ void row_dot(uint8_t* sm8, uint32_t n_cols, uint32_t n_tiles, uint32_t spin, uint32_t* err,
-                                        ColFn col, WeightFn weight, BeginFn begin, WordFn word, RowsFn rows) {
+__device__ __forceinline__ uint32_t row_dot(uint8_t* sm8, uint32_t n_cols, uint32_t n_tiles, uint32_t spin,
+                                            uint32_t* err, ColFn col, WeightFn weight, BeginFn begin, WordFn word,
+                                            RowsFn rows) {
   uint8_t* opA = sm8;
   uint8_t* opB = sm8 + 4 * kUmmaOperand;
   DotSync* sy = reinterpret_cast<DotSync*>(opB + dot_stages(n_cols) * kDotStage);
@@ -98,6 +100,7 @@ __device__ __forceinline__ void row_dot(uint8_t* sm8, uint32_t n_cols, uint32_t 
   __syncthreads();
   const uint32_t tmem = sy->tmem;
   bool ok = true;
+  uint32_t left = blockIdx.x;  // first tile without its sums
   uint32_t g = 0;  // chunks so far: chunk g uses half g & 1, its products complete phase g >> 1 of bar[g & 1]
   for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     begin();
@@ -147,7 +150,10 @@ __device__ __forceinline__ void row_dot(uint8_t* sm8, uint32_t n_cols, uint32_t 
       tmem_ld_wait(d);
       s[r] = {umma_value(d), umma_value(d + 4), umma_value(d + 8), umma_value(d + 12)};
     }
-    if (ok) rows(tile, s);
+    if (ok) {
+      rows(tile, s);
+      left = tile + gridDim.x;
+    }
   }
   if (!ok) {
     if (tid == 0) {
@@ -159,6 +165,7 @@ __device__ __forceinline__ void row_dot(uint8_t* sm8, uint32_t n_cols, uint32_t 
   umma_fence_before();
   __syncthreads();
   if (tid < 32) tmem_free<4 * kDotCols>(tmem);
+  return left;
 }
 
 // Persistent grid: as many blocks as are resident at once, never more blocks

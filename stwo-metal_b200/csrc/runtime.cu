@@ -9,23 +9,6 @@
 
 namespace stwo_b200 {
 std::atomic<uint64_t> g_kernel_launches{0};
-
-static std::atomic<uint32_t*> g_fault_word{nullptr};
-uint32_t* fault_word() { return g_fault_word.load(std::memory_order_acquire); }
-bool take_fault() {
-  uint32_t* w = fault_word();
-  return w && __atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL) != 0;
-}
-static cudaError_t make_fault_word() {
-  if (fault_word()) return cudaSuccess;
-  uint32_t* w = nullptr;
-  const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&w), sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
-  if (e != cudaSuccess) return e;
-  *w = 0;
-  uint32_t* none = nullptr;
-  if (!g_fault_word.compare_exchange_strong(none, w)) cudaFreeHost(w);  // another thread was first
-  return cudaSuccess;
-}
 }  // namespace stwo_b200
 
 using namespace stwo_b200;
@@ -52,7 +35,6 @@ int stwo_b200_init(int device, char* err, size_t err_len) {
   STWO_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, device));
   uint64_t threshold = UINT64_MAX;
   STWO_CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold));
-  STWO_CUDA_TRY(make_fault_word());
   return ok(err, err_len);
 }
 
@@ -104,7 +86,6 @@ int stwo_b200_stream_destroy(void* stream, char* err, size_t err_len) {
 
 int stwo_b200_stream_sync(void* stream, char* err, size_t err_len) {
   STWO_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
-  if (take_fault()) return set_err(err, err_len, STWO_B200_ETIMEOUT, "a tensor-core product did not complete in time");
   return ok(err, err_len);
 }
 
