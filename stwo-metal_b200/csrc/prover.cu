@@ -393,10 +393,21 @@ uint32_t poly_eval_chunks(uint32_t lg) { return lg > 10 ? 1u << (lg - 10) : 1u; 
 // buckets per polynomial and a w_hi table of at most 2^14 entries).
 uint32_t poly_eval_lo_bits(uint32_t lg) { return lg >= 13 && lg <= 24 ? kEvalLoBits : lg / 2; }
 
-// From 32 polynomials up the tensor-core form (its cost is that of a whole group
-// of 128): 108 polynomials of 2^20 119 -> 82 us.  Below, most of a product's
-// rows would be empty.
-constexpr uint32_t kEvalDotPolys = 32;
+// Whether the tensor-core form is the faster one for these sizes.  Both take
+// whole rounds of the chip: the bucket kernel 8.2 us for every 148 blocks (8
+// units each), the tensor-core form 6 us for a bucket of a block, however few
+// rows of its products are polynomials, 0.05 us for every polynomial of a group
+// and 2.4 us more to begin with.  Measured with cold caches (us, tensor cores / buckets): 2^13 to 2^15,
+// 32 to 200 polynomials 15 to 18 / 14 to 15; 2^16 128 18 / 16, 160 19 / 23; 2^18
+// 32 26 / 16, 64 29 / 24, 96 33 / 34, 160 57 / 53, 200 60 / 62; 2^20 32 74 / 43,
+// 64 80 / 71, 96 92 / 106, 108 97 / 116, 129 162 / 134, 192 170 / 195; 2^22 64
+// 284 / 257, 80 294 / 319, 128 361 / 504.  At none of the 300 sizes timed (2^13
+// to 2^24, 32 to 1024 polynomials) is the form taken more than 2% the slower one.
+bool eval_dot_is_faster(uint32_t n_polys, uint32_t buckets, uint32_t groups, uint32_t blocks) {
+  const uint64_t units = (uint64_t)n_polys * (buckets / kEvalUnitBuckets);
+  const uint64_t bucket_rounds = (units + 8 * 148 - 1) / (8 * 148), dot_rounds = (buckets + blocks - 1) / blocks;
+  return 240 + dot_rounds * (600 + 5 * n_polys / groups) < 820 * bucket_rounds;  // in 10 ns
+}
 int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg, const qm31* d_w_lo,
                      const qm31* d_w_hi, qm31* d_partial, qm31* d_out, uint32_t* fault, uint32_t spin, cudaStream_t s,
                      char* err, size_t err_len) {
@@ -412,11 +423,11 @@ int launch_poly_eval(const uint32_t* const* polys, uint32_t n_polys, uint32_t lg
     // 2^(lg - h) >= kEvalUnitBuckets buckets of 1024 indices per polynomial
     const uint32_t units_per_poly = (1u << (lg - h)) / kEvalUnitBuckets;
     const uint32_t units = n_polys * units_per_poly;
-    if (n_polys >= kEvalDotPolys) {
+    const uint32_t groups = (n_polys + 127) / 128, buckets = 1u << (lg - h);
+    const uint32_t blocks = std::min(buckets, std::max(1u, 148u / groups));
+    if (eval_dot_is_faster(n_polys, buckets, groups, blocks)) {
       static std::atomic<uint32_t> attr{0};
       STWO_CUDA_TRY(ensure_smem_limit(poly_eval_dot_kernel, (int)kEvalDotSmem, attr));
-      const uint32_t groups = (n_polys + 127) / 128, buckets = 1u << (lg - h);
-      const uint32_t blocks = std::min(buckets, std::max(1u, 148u / groups));
       poly_eval_dot_kernel<<<dim3(blocks, groups), 256, kEvalDotSmem, s>>>(pt, n_polys, buckets, d_w_lo, d_w_hi,
                                                                            d_partial, fault, spin);
       STWO_CHECK_LAUNCH();

@@ -62,10 +62,18 @@ def test_numerators_alignment(oracle, in_off, out_off):
         assert (o.buf.to_host()[out_off:] == r).all()
 
 
-@pytest.mark.parametrize("log_n", [12, 13, 14, 17])
-@pytest.mark.parametrize("n_polys", [1, 31, 32, 33, 127, 128, 129, 300])
+# 2^12 takes the chunked kernel; the tensor cores (whole groups of 128, short
+# ones, several buckets a block) and the bucket kernel on both sides of the line
+BATCH_EVAL = [(12, n) for n in (1, 31, 32, 33, 127, 128, 129, 300)]
+BATCH_EVAL += [(13, n) for n in (1, 31, 32, 33, 127, 128, 129, 300, 1024)]
+BATCH_EVAL += [(14, n) for n in (1, 31, 32, 33, 127, 128, 129, 300, 600, 1024)]
+BATCH_EVAL += [(15, 300), (16, 148), (16, 149), (16, 256), (16, 257)]
+BATCH_EVAL += [(17, n) for n in (1, 31, 32, 33, 74, 75, 76, 127, 128, 129, 149, 300)]
+BATCH_EVAL += [(18, 74), (18, 76), (18, 128), (18, 129), (19, 96), (19, 260)]
+
+
+@pytest.mark.parametrize("log_n,n_polys", BATCH_EVAL)
 def test_batch_eval_groups(oracle, log_n, n_polys):
-    # 2^12 takes the chunked kernel, from 2^13 up 32 polynomials or more the tensor cores
     rng = np.random.default_rng(1000 * log_n + n_polys)
     polys = [words(rng, 1 << log_n) for _ in range(min(n_polys, 9))]
     polys[0][:] = P
