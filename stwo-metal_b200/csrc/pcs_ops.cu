@@ -98,9 +98,14 @@ __global__ void __launch_bounds__(256) numerators_kernel(NumeratorTerms t, uint3
 }
 
 // The same sums on the tensor cores (rowdot.cuh): whole 512-row tiles, columns
-// and outputs 16-byte aligned.  The call returns before the kernel has run, so
+// and outputs 16-byte aligned, and three terms or more: below, the operands'
+// preparation costs more than the products save (us, tensor cores / integer
+// pipes, cold caches: one term 3.4 / 2.2 at 2^9 and 5.6 / 4.5 at 2^18, two 3.5 /
+// 2.8 and 5.8 / 5.1, three 3.5 / 3.6 and 5.7 / 5.8, seven 3.6 / 5.6 and 6.4 /
+// 8.4; 107 at 2^20 99 / 161).  The call returns before the kernel has run, so
 // a wait that gives up has nobody to report to: its thread takes the rows it
 // is left with on the integer pipes.
+constexpr uint32_t kNumDotTerms = 3;
 __global__ void __launch_bounds__(kDotThreads, kDotBlocks) numerators_dot_kernel(NumeratorTerms t, uint32_t n_terms,
                                                                        qm31 b_sum, uint64_t n, int accumulate,
                                                                        Col4 out, uint32_t spin) {
@@ -386,7 +391,7 @@ extern "C" int stwo_b200_accumulate_numerators_polls(const uint32_t* const* d_co
         aligned = aligned && reinterpret_cast<uintptr_t>(t.col[k]) % 16 == 0;
       }
       const int acc = k0 > 0 ? 1 : 0;
-      bool dot = aligned && n % kDotRows == 0 && nt > 0;
+      bool dot = aligned && n % kDotRows == 0 && nt >= kNumDotTerms;
       for (int k = 0; k < 4; k++) dot = dot && reinterpret_cast<uintptr_t>(out.c[k]) % 16 == 0;
       if (dot) {
         static std::atomic<uint32_t> attr{0};

@@ -26,7 +26,7 @@ def words(rng, n):
 
 
 @pytest.mark.parametrize("log_n", [8, 9, 10, 13])
-@pytest.mark.parametrize("n_terms", [1, 7, 8, 9, 16, 17, 31, 33, 48, 255, 257])
+@pytest.mark.parametrize("n_terms", [1, 2, 3, 7, 8, 9, 16, 17, 31, 33, 48, 255, 257, 258, 259])
 def test_numerators_tiles_and_chunks(oracle, log_n, n_terms):
     rng = np.random.default_rng(100 * log_n + n_terms)
     cols = [words(rng, 1 << log_n) for _ in range(min(n_terms, 20))]
