@@ -54,7 +54,8 @@ __global__ void wide_fib_trace_kernel(const uint32_t* __restrict__ a, const uint
 // Four consecutive points per thread: 16-byte loads keep four times the bytes
 // in flight per load, which this memory-latency-bound loop needs.
 // n_points % 4 == 0, columns 16-byte aligned.  The tensor-core form
-// composition_dot_kernel takes every domain of at least one 512-row tile.
+// composition_dot_kernel takes every domain of at least one 512-row tile from
+// kCompositionDotCols columns on.
 __global__ void __launch_bounds__(256) composition4_kernel(const uint32_t* __restrict__ evals, uint64_t col_stride,
                                                           uint32_t n_cons, const qm31* __restrict__ powers,
                                                           const uint32_t* __restrict__ denom_inv, uint32_t log_n,
@@ -561,6 +562,13 @@ __global__ void __launch_bounds__(256) quotient4_kernel(QuotientParams q, PolyTa
 // ---- the row kernels on the tensor cores (rowdot.cuh) ----
 // 512-row tiles, four consecutive rows a thread, the sums over the columns as
 // 8-bit products.  Same values as composition4_kernel / quotient4_kernel.
+// From 6 columns on the composition takes this form.  Below, a tile's fixed work
+// is most of it, and composition4_kernel is the faster one (us, tensor cores /
+// integer pipes: 3 columns 4.2 / 2.9 at 2^10 points, 17.1 / 10.4 at 2^20, 59.5 /
+// 37.8 at 2^22; 5 columns 4.2 / 3.7, 17.4 / 15.0, 60.0 / 55.7; 6 columns 4.0 /
+// 3.8, 17.7 / 17.8, 60.5 / 64.6; 16 columns 4.1 / 6.2, 25.3 / 38.1, 83 / 123).
+// The quotients have 8 columns more, 11 or more in all, and gain at every size.
+constexpr uint32_t kCompositionDotCols = 6;
 constexpr uint32_t kArrivalsWord = 9;   // word of the same buffer that the tree launches count their blocks in
 constexpr uint32_t kStreamErrWord = 8;  // word of the prover's flag buffer set by a wait that ran out
 
@@ -2268,7 +2276,7 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     comp_stride = 1ull << eval_log;
   }
   const uint64_t n_eval = 1ull << eval_log;
-  if (n_eval % kDotRows == 0 && N <= kDotMaxCols && comp_stride % 4 == 0 &&
+  if (n_eval % kDotRows == 0 && N >= kCompositionDotCols && N <= kDotMaxCols && comp_stride % 4 == 0 &&
       reinterpret_cast<uintptr_t>(comp_src) % 16 == 0)
     composition_dot_kernel<<<dot_grid(dot_smem(N), 0, (uint32_t)(n_eval / kDotRows)), kDotThreads,
                              dot_smem(N), s>>>(comp_src, comp_stride, n_cons, d_small, d_denom, log_n, n_eval, d_comp,
