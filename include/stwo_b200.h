@@ -496,8 +496,8 @@ int stwo_b200_prover_set_timing(stwo_b200_prover* prover, int enable, char* err,
 int stwo_b200_prover_phase_times(stwo_b200_prover* prover, double* ms_out, uint32_t n, uint32_t* proofs, char* err,
                                  size_t err_len);
 
-/* Wait bound of the prover's column-streaming kernels (composition,
- * quotients): a thread polls the mbarrier of its block's tensor-core products
+/* Wait bound of the prover's column-streaming kernels (composition, OODS
+ * sums, quotients): a thread polls the mbarrier of its block's tensor-core products
  * at most `polls` times before it gives up, sets the prover's error flag and
  * stores nothing more; the prove then returns STWO_B200_ETIMEOUT.  0 gives up
  * at the first wait (every such prove fails); STWO_B200_STREAM_SPIN_DEFAULT

@@ -1689,8 +1689,9 @@ enum Phase {
 class WideFibProver {
  public:
   bool timing = false;
-  // Polls a consumer of the column-streaming kernels makes before a stage
-  // wait gives up (stwo_b200_prover_set_stream_spin).
+  // Polls that a thread of the column-streaming kernels (composition, OODS
+  // sums, quotients) makes before its wait for a product gives up
+  // (stwo_b200_prover_set_stream_spin).
   uint32_t stream_spin = kStreamSpin;
   std::vector<cudaEvent_t> ev_pool;
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
@@ -2327,7 +2328,7 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     for (int k = 0; k < 8; k++) polys.push_back(split[k]);
     d_vals = d_small + n_w;
     if ((rc = launch_poly_eval(polys.data(), np, lg, d_small, d_small + (1u << h), d_oods_partial, d_vals,
-                               d_found + kStreamErrWord, kStreamSpin, s, err, err_len)))
+                               d_found + kStreamErrWord, stream_spin, s, err, err_len)))
       return rc;
   }
 
@@ -2413,10 +2414,10 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
       cudaStreamSynchronize(s);
       return set_err(err, err_len, code, "%s", what);
     };
-    // A timed-out composition stream leaves partial rows behind: report it
-    // before any check of the values built on them.
+    // A wait that gave up leaves rows or sums out: report it before any check
+    // of the values built on them.
     if (*reinterpret_cast<const uint32_t*>(h_tx + tx_flag_off))
-      return fail(STWO_B200_ETIMEOUT, "column stream: a bulk copy did not complete in time");
+      return fail(STWO_B200_ETIMEOUT, "column stream: a tensor-core product did not complete in time");
     ch.mix_root(root1);
     const qm31 random_coeff = ch.draw_secure_felt();
     if (!qm31_eq(random_coeff, fs.random_coeff))
@@ -2503,10 +2504,10 @@ int WideFibProver::prove_body(const uint32_t* d_a, const uint32_t* d_b, ProofOut
     STWO_CHECK_LAUNCH();
     STWO_CUDA_TRY(cudaStreamSynchronize(s));
     const DevChannel* dc = reinterpret_cast<const DevChannel*>(hp + chan_off);
-    // A timed-out stream leaves the transcript built on partial rows, so its
+    // A wait that gave up leaves the transcript built on partial rows, so its
     // flag is reported first.
     if (*reinterpret_cast<const uint32_t*>(hp + flag_off))
-      return set_err(err, err_len, STWO_B200_ETIMEOUT, "column stream: a bulk copy did not complete in time");
+      return set_err(err, err_len, STWO_B200_ETIMEOUT, "column stream: a tensor-core product did not complete in time");
     if (dc->error) return set_err(err, err_len, STWO_B200_ESTATE, "device channel: draw retry bound exhausted");
     dev_ch.set_state(dc->digest, dc->n_draws);
     std::memcpy(fri_end_digest, dc->digest, 32);

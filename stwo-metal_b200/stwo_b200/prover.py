@@ -85,8 +85,8 @@ class WideFibProver:
 
     def set_stream_spin(self, polls: int) -> None:
         """Poll bound of a thread's wait for its block's products in the
-        column-streaming kernels (composition, quotients); 0 makes every such
-        wait give up at once, so the prove returns STWO_B200_ETIMEOUT."""
+        column-streaming kernels (composition, OODS sums, quotients); 0 makes
+        every such wait give up at once, so the prove returns STWO_B200_ETIMEOUT."""
         ffi.call("stwo_b200_prover_set_stream_spin", self.handle, C.c_uint32(polls))
 
     def close(self):

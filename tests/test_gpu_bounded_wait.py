@@ -1,12 +1,12 @@
-"""The bounded device waits of the column-streaming kernels give up cleanly.
+"""The bounded device waits of the tensor-core kernels give up cleanly.
 
-The composition and quotient kernels stream columns through a shared-memory
-ring whose stages complete on mbarriers; every wait on them is bounded.  Here
-the consumers' bound is set to zero polls, so the first stage wait of every
-block runs out: the block sets the prover's error flag, the producer waits for
-its copies already in flight and leaves, and the prove returns
-STWO_B200_ETIMEOUT with a message.  Nothing faults, and the same prover then
-proves the same inputs with the default bound, byte for byte as the oracle.
+The composition, OODS and quotient kernels wait on mbarriers for their blocks'
+tensor-core products; every wait polls a bounded number of times.  Here the
+bound is set to zero polls, so the first wait of every thread runs out: the
+kernel sets the prover's error flag, stores no more rows, waits for the products
+still in flight and leaves, and the prove returns STWO_B200_ETIMEOUT with a
+message.  Nothing faults, and the same prover then proves the same inputs with
+the default bound, byte for byte as the oracle.
 """
 import ctypes as C
 
