@@ -36,23 +36,14 @@ __host__ __device__ __forceinline__ uint32_t m31_mul_tw2(uint32_t b, uint32_t t2
 }
 __host__ __device__ __forceinline__ uint32_t m31_mul(uint32_t a, uint32_t b) { return m31_mul_tw2(a, b << 1); }
 __host__ __device__ __forceinline__ uint32_t m31_sqr(uint32_t a) { return m31_mul(a, a); }
-__host__ __device__ inline uint32_t m31_pow(uint32_t a, uint64_t e) {
-  uint32_t r = 1;
-  while (e) {
-    if (e & 1) r = m31_mul(r, a);
-    a = m31_mul(a, a);
-    e >>= 1;
-  }
-  return r;
-}
 template <int N>
 __host__ __device__ __forceinline__ uint32_t m31_sqr_n(uint32_t a) {
   for (int i = 0; i < N; i++) a = m31_sqr(a);
   return a;
 }
 // a^(P - 2) by an addition chain on P - 2 = 128 (2^24 - 1) + 125: 30 squarings
-// and 7 products in place of the 30 squarings and 29 products of m31_pow, all
-// of them one dependent chain in the row kernels' epilogues.  0 -> 0.
+// and 7 products in place of the 30 squarings and 29 products of the binary method,
+// all of them one dependent chain in the row kernels' epilogues.  0 -> 0.
 __host__ __device__ inline uint32_t m31_inv(uint32_t a) {
   const uint32_t e5 = m31_mul(m31_sqr_n<2>(a), a);
   const uint32_t e15 = m31_mul(m31_sqr(e5), e5);

@@ -2140,13 +2140,6 @@ class WideFibProver {
     return 0;
   }
 
-  int download_root(const MerkleTree& t, Hash32& root, char* err, size_t err_len) {
-    STWO_CUDA_TRY(cudaMemcpyAsync(h_pinned, t.layer(0), 32, cudaMemcpyDeviceToHost, s));
-    STWO_CUDA_TRY(cudaStreamSynchronize(s));
-    std::memcpy(root.data(), h_pinned, 32);
-    return 0;
-  }
-
   int commit_columns(uint32_t* const* cols, const std::vector<uint32_t>& logs, MerkleTree& t, char* err,
                      size_t err_len) {
     std::vector<uint8_t*> layers(t.L + 1);
@@ -2843,8 +2836,6 @@ struct SeededFriProver {
   std::vector<void*> allocs;
   qm31* d_alphas = nullptr;  // the folding alphas (uploaded per call; read by the fold kernels)
   qm31* h_alphas = nullptr;  // pinned staging of the alphas
-  uint64_t* d_gather_addr = nullptr;
-  uint8_t* d_gather_out = nullptr;
   size_t gather_cap = 0;     // entries (words or hashes)
   uint8_t* h_stage = nullptr;  // pinned: addresses (8 B / entry), then gathered bytes (32 B / entry)
   uint32_t* d_arrivals = nullptr;  // a word for each tree: they are built side by side
