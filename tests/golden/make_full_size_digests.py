@@ -9,6 +9,7 @@ SHA-256 of its proof bytes (proofs):
 - commit_plain: 32 columns of log 16 (numpy PCG64 seed 1001), natural order,
   blowup 1, lifted Blake2s tree of log 17;
 - wide_fib_prove: 100 columns x 2^20 rows (seed 2), default PcsConfig;
+- wide_fib_narrow: 3 columns x 2^23 rows (seed 23), default PcsConfig;
 - commit_uneven: 512 columns, log sizes U{12..22} (seed 3), values seed 1003,
   blowup 2, lifted tree of log 24;
 - fri_heavy: one QM31 column of log 24 (seed 4), 70 query draws.
@@ -17,7 +18,8 @@ bench.py compares its roots and proofs at these sizes with these digests, so
 that a bench line states bit-exactness without running the oracle for
 minutes.  tests/test_golden.py checks the cheap entries against the oracle
 again; tests/test_gpu_full_size.py checks every one of them on the GPU
-against a fresh oracle run.
+against a fresh oracle run, but wide_fib_narrow, whose GPU proof
+tests/test_gpu_row_kernels.py compares with the digest.
 """
 import hashlib
 import json
@@ -48,6 +50,11 @@ def wide_fib_columns():
     return r.integers(0, P, 1 << 20, dtype=np.uint32), r.integers(0, P, 1 << 20, dtype=np.uint32)
 
 
+def wide_fib_narrow_columns():
+    r = np.random.default_rng(23)
+    return r.integers(0, P, 1 << 23, dtype=np.uint32), r.integers(0, P, 1 << 23, dtype=np.uint32)
+
+
 def commit_root(oracle, logs, cols, blowup, natural):
     L = max(logs) + blowup
     init, lg = oracle.canonic_half_coset_root(L + 1)
@@ -74,6 +81,10 @@ def main():
     proof = oracle.prove_wide_fib(oracle.wide_fib_config(20, 100), a, b)
     out["wide_fib_prove_sha256"] = hashlib.sha256(proof).hexdigest()
     out["wide_fib_prove_bytes"] = len(proof)
+    a, b = wide_fib_narrow_columns()
+    proof = oracle.prove_wide_fib(oracle.wide_fib_config(23, 3), a, b)
+    out["wide_fib_narrow_sha256"] = hashlib.sha256(proof).hexdigest()
+    out["wide_fib_narrow_bytes"] = len(proof)
     coords, alphas, queries = oracle.fri_inputs(24, 4, 70)
     fri = oracle.fri_prove_seeded(coords, 24, alphas, queries)
     out["fri_heavy_sha256"] = hashlib.sha256(fri).hexdigest()
