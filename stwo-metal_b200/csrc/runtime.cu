@@ -9,6 +9,21 @@
 
 namespace stwo_b200 {
 std::atomic<uint64_t> g_kernel_launches{0};
+
+// One small page-locked allocation, made by the first init and kept until the
+// process ends.  While one lives, the driver keeps the chunk that it takes small
+// page-locked allocations from; without it every prover that is made and closed
+// maps and unmaps that chunk (making a FRI prover of 2^24: 9.4 ms, with it 6.8).
+static cudaError_t keep_pinned_chunk() {
+  static std::atomic<void*> kept{nullptr};
+  if (kept.load(std::memory_order_acquire)) return cudaSuccess;
+  void* p = nullptr;
+  const cudaError_t e = cudaHostAlloc(&p, 64, cudaHostAllocPortable);
+  if (e != cudaSuccess) return e;
+  void* none = nullptr;
+  if (!kept.compare_exchange_strong(none, p)) cudaFreeHost(p);  // another thread was first
+  return cudaSuccess;
+}
 }  // namespace stwo_b200
 
 using namespace stwo_b200;
@@ -35,6 +50,7 @@ int stwo_b200_init(int device, char* err, size_t err_len) {
   STWO_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, device));
   uint64_t threshold = UINT64_MAX;
   STWO_CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold));
+  STWO_CUDA_TRY(keep_pinned_chunk());
   return ok(err, err_len);
 }
 
