@@ -490,7 +490,8 @@ int stwo_b200_prover_footprint(const stwo_b200_wide_fib_config* cfg, size_t* dev
  * 4 composition, 5 composition interpolate, 6 composition evaluate,
  * 7 composition Merkle, 8 OODS sampling, 9 FRI quotients, 10 FRI Merkle,
  * 11 FRI folds, 12 grind, 13 decommit (each phase spans to the next one,
- * host channel work included).  No reference counterpart (the reference's
+ * host channel work included; FRI layers of up to 2^16 values are one launch
+ * from the fold to the channel step, counted as FRI Merkle).  No reference counterpart (the reference's
  * env-gated timers STWO_METAL_PROFILE_* play this role). */
 int stwo_b200_prover_set_timing(stwo_b200_prover* prover, int enable, char* err, size_t err_len);
 int stwo_b200_prover_phase_times(stwo_b200_prover* prover, double* ms_out, uint32_t n, uint32_t* proofs, char* err,

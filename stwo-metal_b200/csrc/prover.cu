@@ -618,7 +618,8 @@ __global__ void __launch_bounds__(kDotThreads, kDotBlocks) composition_dot_kerne
 // Bit k of the tile's number is bit log-1-b-k of J0: B is the sum of one entry
 // of each of two tables over 7 bits of it, built by the block, and of the
 // steps of its bits above 14 (domains above 2^23).  A third table would keep a
-// third block off the SM (100 columns: 75 KB of shared memory each).
+// third block off the SM (100 columns: 75 KB of shared memory each).  Above 128
+// columns two blocks fit with either; the table's bits are the same there.
 constexpr uint32_t kTileTabBits = 7, kTileTabs = 2;
 static_assert((1 << kTileTabBits) == kDotThreads, "thread e builds entry e of each table");
 __global__ void __launch_bounds__(kDotThreads, kDotBlocks) quotient_dot_kernel(QuotientParams q, PolyTable cols,
@@ -1450,10 +1451,12 @@ __global__ void __launch_bounds__(kTreeThreads) fri_nodes_kernel(const uint8_t* 
 // that makes it (of the circle evaluation, or of the layer before it), its
 // leaves, its tree, the root's mix and the draw of its alpha, one value a
 // thread.  Larger layers fold with wide loads and hash several levels a thread
-// first.  Against a launch each for the fold, the lower levels and the top with
-// the channel: layers of 2^15 30 -> 25 us, of 2^10 23 -> 18 us with the gaps, but
-// of 2^16 32 -> 41 us (512 blocks of mostly one busy warp); the whole proofs were
-// timed with 16 here, 173 x 2^17 1339 -> 1271 us, and with 17, 30 us slower.
+// first.  Against three launches, for the fold, the lower levels and the top with
+// the channel, layers of 2^15 took 30 -> 25 us and of 2^10 23 -> 18 us with the
+// gaps.  Against the two launches that larger layers take now (the fold, then
+// fri_nodes_kernel), one of 2^16 is 37 us of 512 blocks of mostly one busy warp,
+// or 8 and 27 us and a gap: proofs take the same with 15 here (173 x 2^17 1294 and
+// 1295 us, 100 x 2^20 3815 and 3813).
 constexpr uint32_t kFriLayerLog = 16;
 static_assert(kFriLayerLog <= kTreeLastLog + 7, "the last block stages one hash for each block of 2^7 values");
 template <bool CIRCLE>

@@ -10,10 +10,12 @@
 // their folds; here it takes a quarter of a 16-byte load and of a 16-byte
 // shared store.  What is left is the memory time of the columns, the latency of
 // a chunk's loads (12 warps an SM) and the arithmetic of a tile's rows.
-// Measured at 100 x 2^21 (with 8 more columns for the quotients), against the
-// integer-pipe kernels on a shared-memory ring: composition 283 -> 195 us,
-// quotients 240 -> 190 us (4.6 TB/s); numerators of 107 terms at 2^20 168 ->
-// 107 us.
+// Measured against the integer-pipe kernels on a shared-memory ring: composition
+// of 100 columns of 2^21 points 283 -> 195 us (0.87 GB, 4.5 TB/s), quotients of
+// 108 240 -> 190 us (0.94 GB, 4.9 TB/s), numerators of 107 terms at 2^20 168 ->
+// 107 us.  Above 160 columns (the quotients, with their tables: 128) the weights
+// leave room for two blocks an SM, quotients of 264 columns of 2^20 points 264 ->
+// 191 us; above 768 (736) for one, 1024 columns of 2^18 points 265 -> 277 us.
 //
 // A block of 128 threads owns 512 consecutive rows, thread t rows 4t..4t+3:
 // it loads 16 bytes of each of 16 columns, and row 4t + r of 4 of them is one
